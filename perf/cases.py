@@ -110,7 +110,7 @@ def draw(rng: random.Random):
         return _grid(None, "mhd", _box(rng, 3, 32, 112), precision, "run", rng.randint(5, 10),
                      limiter=rng.choice(["mc", "vl"]), sides=rng.choice(["outflow", "mirror"]))
     kind = rng.choice(["ensemble", "serving"])
-    hi = rng.randint(128, 400) if kind == "ensemble" else rng.randint(40, 80)
+    hi = rng.randint(128, 400) if kind == "ensemble" else rng.randint(40, 72)
     return _batch(None, kind, rng.randint(16, 96), 64 if kind == "ensemble" else 24, hi,
                   rng.randint(5, 25), rng.randint(2, 1 << 20))
 
