@@ -568,10 +568,12 @@ int gp_batch_add(gp_batch* b, const gp_grid_desc* grid, const gp_scheme* scheme,
         a.Bsout[q] = on ? B[stage == 1 ? b1 : b2][q] : nullptr;
         a.Ee[q] = Ee[q];
         a.dx[q] = s.dx[q];
+        a.inv_dx[q] = gp::fixed_inv(s.dx[q]);
         for (int r = 0; r < 6; r++) a.ct[q][r] = static_cast<double*>(ct[q][r]);
       }
       a.dtdx = sc->dtdx;
       a.gamma = scheme->gamma;
+      a.inv_gm1 = gp::fixed_inv(scheme->gamma - 1.0);
       a.small_rho = scheme->small_rho;
       a.small_prs = scheme->small_prs;
       a.stage = stage;

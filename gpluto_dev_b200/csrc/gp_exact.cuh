@@ -1,0 +1,130 @@
+// gp_exact.cuh -- correctly rounded FP64 division and square root without
+// branches, for the Riemann solvers (sm_100a).
+//
+// The reference's bits need every quotient and root correctly rounded.  The
+// language's operators give that, but each one carries its own range test
+// and branch, so a solver with some forty of them is a chain of short basic
+// blocks whose latencies do not overlap, and quotients with a common divisor
+// repeat the divisor's reciprocal.  Here the range test is only accumulated
+// in a flag (`bad`), the arithmetic is straight-line, and the caller redoes
+// the few faces whose flag is set with the operators.
+//
+// Methods (published): Newton's iteration on the reciprocal and the
+// correction of a quotient by its exact remainder, P. Markstein, "Computation
+// of elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34 (1990); division by a divisor whose correctly rounded reciprocal is
+// known in one product and two FMAs, N. Brisebarre, J.-M. Muller, S. K.
+// Raina, IEEE Trans. Comput. 53 (2004).  The seeds are PTX's rcp.approx.ftz.f64
+// and rsqrt.approx.ftz.f64.
+//   * y1 = y0 + y0 (e + e^2), e = 1 - b y0, is 1/b to 2^-58; one more Newton
+//     step from there rounds correctly (Markstein), also for the all-ones
+//     significand that his theorem leaves out once y1 is rounded upwards:
+//     1/b then lies just above a midpoint, and only y1 = the lower neighbour
+//     would take the step to it.
+//   * q = a y, q + y (a - b q) with y = RN(1/b) is RN(a/b) (no exception while
+//     nothing under- or overflows).
+//   * s + h (a - s^2), s = a y, h = y/2 with y within 0.55 ulp of a^(-1/2) is
+//     RN(sqrt(a)).
+// All three hold for every significand of 4 to 12 bits (checked exhaustively)
+// and agree with the operators on the arguments of tests/test_gpu_exact.py.
+#pragma once
+#include <cstdint>
+#include <cuda_runtime.h>
+
+namespace gp {
+
+// The language's operators (FP32 of the mixed form; FP64 where a face left
+// the range of FastArith).
+template <typename R>
+struct PlainArith {
+  static constexpr bool FAST = false;
+  __device__ __forceinline__ R inv(R b) { return R(1) / b; }
+  __device__ __forceinline__ R inv_pos(R b) { return R(1) / b; }
+  __device__ __forceinline__ R quot(R a, R b, R) { return a / b; }
+  __device__ __forceinline__ R quot_pos(R a, R b, R) { return a / b; }
+  __device__ __forceinline__ R div(R a, R b) { return a / b; }
+  __device__ __forceinline__ R div_pos(R a, R b) { return a / b; }
+  __device__ __forceinline__ R root(R a) { return sqrt(a); }
+  __device__ __forceinline__ R root0(R a) { return sqrt(a); }
+};
+
+struct FastArith {
+  static constexpr bool FAST = true;
+  bool bad = false;
+
+  // |b| in [2^-200, 2^200]: no intermediate of inv or quot leaves the normal
+  // range when the dividend is 0 or in [2^-700, 2^700]
+  static constexpr unsigned kDivLo = (1023u - 200u) << 20, kDivSpan = 400u << 20;
+  static constexpr unsigned kNumLo = (1023u - 700u) << 20, kNumSpan = 1400u << 20;
+  // root: a in [2^-400, 2^400]
+  static constexpr unsigned kRootLo = (1023u - 400u) << 20, kRootSpan = 800u << 20;
+
+  // RN(1/b), b > 0 (a negative b sets the flag)
+  __device__ __forceinline__ double inv_pos(double b) {
+    bad |= (unsigned)__double2hiint(b) - kDivLo > kDivSpan;
+    double y0;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(b));
+    const double e = __fma_rn(-b, y0, 1.0);
+    const double y1 = __fma_ru(__fma_rn(e, e, e), y0, y0);
+    return __fma_rn(__fma_rn(-b, y1, 1.0), y1, y1);
+  }
+  // RN(1/b)
+  __device__ __forceinline__ double inv(double b) {
+    const int hi = __double2hiint(b), s = hi & (int)0x80000000;
+    const double y = inv_pos(__hiloint2double(hi & 0x7fffffff, __double2loint(b)));
+    return __hiloint2double(__double2hiint(y) | s, __double2loint(y));
+  }
+  // RN(a/b) with y = inv(b); a zero keeps the sign the operator gives
+  __device__ __forceinline__ double quot(double a, double b, double y) {
+    // a = 0 passes, a denormal does not: its low word is not 0
+    const unsigned lo = (unsigned)__double2loint(a);
+    const unsigned k = ((unsigned)__double2hiint(a) & 0x7fffffffu) | (lo < 1u ? lo : 1u);
+    bad |= (k - kNumLo > kNumSpan) & (k != 0u);
+    const double q = __dmul_rn(a, y);
+    const double p = __fma_rn(__fma_rn(-b, q, a), y, q);
+    const int s = __double2hiint(q) & (int)0x80000000;
+    return __hiloint2double((__double2hiint(p) & 0x7fffffff) | s, __double2loint(p));
+  }
+  // the same for a > 0 and b > 0 (anything else sets the flag)
+  __device__ __forceinline__ double quot_pos(double a, double b, double y) {
+    bad |= (unsigned)__double2hiint(a) - kNumLo > kNumSpan;
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+  }
+  __device__ __forceinline__ double div(double a, double b) { return quot(a, b, inv(b)); }
+  __device__ __forceinline__ double div_pos(double a, double b) { return quot(a, b, inv_pos(b)); }
+  // RN(sqrt(a)), a > 0
+  __device__ __forceinline__ double root(double a) {
+    bad |= (unsigned)__double2hiint(a) - kRootLo > kRootSpan;
+    double y0;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(a));
+    const double e = __fma_rn(-a, __dmul_rn(y0, y0), 1.0);
+    const double y1 = __fma_rn(__dmul_rn(e, __fma_rn(e, 0.375, 0.5)), y0, y0);
+    const double g = __dmul_rn(a, y1);
+    return __fma_rn(__fma_rn(-g, g, a), __dmul_rn(0.5, y1), g);
+  }
+  // root of a >= +0
+  __device__ __forceinline__ double root0(double a) {
+    const bool zero = __double_as_longlong(a) == 0;
+    const double r = root(zero ? 1.0 : a);
+    return zero ? a : r;
+  }
+};
+
+// RN(a/b) for a divisor fixed over a launch, y = RN(1/b) formed once; the
+// operator where the dividend is not 0 or in [2^-700, 2^700].  The caller
+// vouches for b in [2^-200, 2^200] (y = 0 otherwise: the operator).
+__device__ __forceinline__ double fixed_quot(double a, double b, double y) {
+  FastArith f;
+  const double p = f.quot(a, b, y);
+  return (f.bad || y == 0.0) ? a / b : p;
+}
+__device__ __forceinline__ float fixed_quot(float a, float b, float) { return a / b; }
+
+// 1/b for fixed_quot (host side), 0 when b is outside its range
+__host__ __device__ inline double fixed_inv(double b) {
+  const double m = b < 0 ? -b : b;
+  return (m >= 0x1p-200 && m <= 0x1p200) ? 1.0 / b : 0.0;
+}
+
+}  // namespace gp

@@ -68,6 +68,7 @@ struct StageArgs {
   const double* dtdx;     // dt/dx_d (3 values in device memory, set per step)
   double dx[3];
   double gamma, small_rho, small_prs;
+  double inv_dx[3], inv_gm1;  // RN(1/dx_d), RN(1/(gamma-1)) for fixed_quot (0: out of its range)
   int stage;              // 1, 2 (RK2, RK3) or 3 (RK3)
   double w0, w1, wr;      // combine weights of stages >= 2: U = w0 U^n + w1 U_c + wr R
                           // (Src/rk_step.cpp:30-61)
@@ -143,11 +144,13 @@ __device__ __forceinline__ constexpr bool rhs_var(int nv) {
 
 // Riemann dispatch for one interface.
 template <int PHYS, int RS, int CT, int DIR, typename R>
-__device__ __forceinline__ R riemann(const R* vl, const R* vr, R* flux, R gamma, R Bn,
+__device__ __forceinline__ R riemann(const R* vl, const R* vr, R* flux, R gamma, R ygm, R Bn,
                                      CTFace<R>& ct, uint32_t& err) {
   if constexpr (PHYS == PHYS_MHD) {
     R cm;
-    if constexpr (RS == RS_HLLD) cm = mhd_hlld<DIR, CT>(vl, vr, flux, gamma, Bn, ct);
+    if constexpr (RS == RS_HLLD && sizeof(R) == sizeof(double))
+      cm = mhd_hlld_fp64<DIR, CT>(vl, vr, flux, gamma, ygm, Bn, ct);
+    else if constexpr (RS == RS_HLLD) cm = mhd_hlld<DIR, CT>(vl, vr, flux, gamma, Bn, ct);
     else if constexpr (RS == RS_TVDLF) cm = mhd_tvdlf<DIR>(vl, vr, flux, gamma, ct);
     else if constexpr (RS == RS_HLLC) cm = mhd_hllc<DIR>(vl, vr, flux, gamma, ct);
     else cm = mhd_hll<DIR>(vl, vr, flux, gamma, ct);
@@ -167,7 +170,7 @@ __device__ __forceinline__ R riemann(const R* vl, const R* vr, R* flux, R gamma,
     return cm;
   } else if constexpr (PHYS == PHYS_RMHD) {
     if constexpr (sizeof(R) == sizeof(double)) {
-      return rmhd_riemann<DIR, RS>(vl, vr, flux, gamma, ct, err);
+      return rmhd_riemann_fp64<DIR, RS>(vl, vr, flux, gamma, ct, err);
     } else {
       // the relativistic HLLD (secant iteration, quartic speeds, nested
       // con2prim) is not usable in FP32 at Lorentz factors ~10: the mixed
@@ -176,7 +179,7 @@ __device__ __forceinline__ R riemann(const R* vl, const R* vr, R* flux, R gamma,
 #pragma unroll
       for (int nv = 0; nv < 8; nv++) { dl[nv] = vl[nv]; dr[nv] = vr[nv]; }
       CTFace<double> cd;
-      double cm = rmhd_riemann<DIR, RS>(dl, dr, df, (double)gamma, cd, err);
+      double cm = rmhd_riemann_fp64<DIR, RS>(dl, dr, df, (double)gamma, cd, err);
 #pragma unroll
       for (int nv = 0; nv < 8; nv++) flux[nv] = (R)df[nv];
       ct.eb = (R)cd.eb; ct.et = (R)cd.et; ct.aL = (R)cd.aL;
@@ -184,7 +187,9 @@ __device__ __forceinline__ R riemann(const R* vl, const R* vr, R* flux, R gamma,
       return (R)cm;
     }
   } else {
-    if constexpr (RS == RS_HLLC) return hd_hllc<DIR>(vl, vr, flux, gamma);
+    if constexpr (RS == RS_HLLC && sizeof(R) == sizeof(double))
+      return hd_hllc_fp64<DIR>(vl, vr, flux, gamma, ygm);
+    else if constexpr (RS == RS_HLLC) return hd_hllc<DIR>(vl, vr, flux, gamma);
     else if constexpr (RS == RS_TVDLF) return hd_tvdlf<DIR>(vl, vr, flux, gamma);
     else return hd_hll<DIR>(vl, vr, flux, gamma);
   }
@@ -209,7 +214,8 @@ __device__ __forceinline__ void cell_update(const StageArgs<CTT>& a, long long n
     // stored in every stage although only stage 1's CFL maximum reads it
     // (Src/update_stage.cpp:422-435): a store conditional on the stage made
     // the FP64 y/z sweeps 40% slower at 256^3
-    a.Cdt[(long long)dir * n + c] = (CTT)(0.5 * ((double)cml + (double)cmr) / a.dx[dir]);
+    a.Cdt[(long long)dir * n + c] =
+        (CTT)fixed_quot(0.5 * ((double)cml + (double)cmr), a.dx[dir], a.inv_dx[dir]);
   } else {
     // mixed form: the stored difference is FP32, so it is formed in FP32
     // (no widening and narrowing conversions, no FP64 division)
@@ -369,7 +375,7 @@ __device__ __forceinline__ void sweep_x_row_ppm(const StageArgs<CTT>& a, const G
     }
     CTFace<R> ct;
     uint32_t fe = 0;
-    cm = riemann<PHYS, RS, CT, 0>(vL, vR, F, gamma, Bn, ct, fe);
+    cm = riemann<PHYS, RS, CT, 0>(vL, vR, F, gamma, (R)a.inv_gm1, Bn, ct, fe);
 #pragma unroll
     for (int nv = 0; nv < NV; nv++)
       if (act && rhs_var<PHYS, NDIM>(nv) && isnan(F[nv])) fe |= ERR_NAN | ERR_QUIT;
@@ -543,7 +549,7 @@ __device__ __forceinline__ void sweep_x_row_mp5(const StageArgs<CTT>& a, const G
     }
     CTFace<R> ct;
     uint32_t fe = 0;
-    cm = riemann<PHYS, RS, CT, 0>(vL, vR, F, gamma, Bn, ct, fe);
+    cm = riemann<PHYS, RS, CT, 0>(vL, vR, F, gamma, (R)a.inv_gm1, Bn, ct, fe);
 #pragma unroll
     for (int nv = 0; nv < NV; nv++)
       if (act && rhs_var<PHYS, NDIM>(nv) && isnan(F[nv])) fe |= ERR_NAN | ERR_QUIT;
@@ -722,7 +728,7 @@ __device__ __forceinline__ void sweep_x_row(const StageArgs<CTT>& a, const Grid3
     }
     CTFace<R> ct;
     uint32_t fe = 0;
-    cm = riemann<PHYS, RS, CT, 0>(vL, vR, F, gamma, Bn, ct, fe);
+    cm = riemann<PHYS, RS, CT, 0>(vL, vR, F, gamma, (R)a.inv_gm1, Bn, ct, fe);
 #pragma unroll
     for (int nv = 0; nv < NV; nv++)
       if (act && rhs_var<PHYS, NDIM>(nv) && isnan(F[nv])) fe |= ERR_NAN | ERR_QUIT;
@@ -859,7 +865,7 @@ __device__ __forceinline__ void sweep_m_col_ppm(const StageArgs<CTT>& a, const G
       }
       CTFace<R> ct;
       uint32_t fe = 0;
-      R cm = riemann<PHYS, RS, CT, DIR>(vL, vR, F, gamma, Bn, ct, fe);
+      R cm = riemann<PHYS, RS, CT, DIR>(vL, vR, F, gamma, (R)a.inv_gm1, Bn, ct, fe);
 #pragma unroll
       for (int nv = 0; nv < NV; nv++)
         if (rhs_var<PHYS, NDIM>(nv) && isnan(F[nv])) fe |= ERR_NAN | ERR_QUIT;
@@ -951,7 +957,7 @@ __device__ __forceinline__ void sweep_m_col_mp5(const StageArgs<CTT>& a, const G
       }
       CTFace<R> ct;
       uint32_t fe = 0;
-      R cm = riemann<PHYS, RS, CT, DIR>(vL, vR, F, gamma, Bn, ct, fe);
+      R cm = riemann<PHYS, RS, CT, DIR>(vL, vR, F, gamma, (R)a.inv_gm1, Bn, ct, fe);
 #pragma unroll
       for (int nv = 0; nv < NV; nv++)
         if (rhs_var<PHYS, NDIM>(nv) && isnan(F[nv])) fe |= ERR_NAN | ERR_QUIT;
@@ -1075,7 +1081,7 @@ __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3
       }
       CTFace<R> ct;
       uint32_t fe = 0;
-      R cm = riemann<PHYS, RS, CT, DIR>(vL, vR, F, gamma, Bn, ct, fe);
+      R cm = riemann<PHYS, RS, CT, DIR>(vL, vR, F, gamma, (R)a.inv_gm1, Bn, ct, fe);
 #pragma unroll
       for (int nv = 0; nv < NV; nv++)
         if (rhs_var<PHYS, NDIM>(nv) && isnan(F[nv])) fe |= ERR_NAN | ERR_QUIT;
@@ -1877,8 +1883,10 @@ __device__ __forceinline__ double finish_cell(const StageArgs<CTT>& a, const Gri
     }
     uint32_t le;
     if constexpr (PHYS == PHYS_MHD) le = mhd_cons2prim(u, v, a.gamma, a.small_rho, a.small_prs);
-    else if constexpr (PHYS == PHYS_RMHD)
-      le = rmhd_cons2prim(u, v, a.gamma, a.small_rho, a.small_prs);
+    else if constexpr (PHYS == PHYS_RMHD) {
+      PlainArith<double> ar;
+      le = rmhd_cons2prim(u, v, a.gamma, a.small_rho, a.small_prs, ar);
+    }
     else le = hd_cons2prim(u, v, a.gamma, a.small_rho, a.small_prs);
     err |= le;
     if (le & ERR_CONS2PRIM_FAIL) err |= ERR_QUIT;

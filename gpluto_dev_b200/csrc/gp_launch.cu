@@ -44,6 +44,7 @@ static StageArgs<CTT> make_args(const StageDesc& d) {
     a.Bsout[q] = d.Bsout[q];
     a.Ee[q] = reinterpret_cast<CTT*>(d.Ee[q]);
     a.dx[q] = d.dx[q];
+    a.inv_dx[q] = fixed_inv(d.dx[q]);
     for (int r = 0; r < 6; r++) a.ct[q][r] = static_cast<CTT*>(d.ct[q][r]);
   }
   a.dtdx = d.dtdx;
@@ -54,6 +55,7 @@ static StageArgs<CTT> make_args(const StageDesc& d) {
   a.Uout = d.Uout;
   a.Vout = d.Vout;
   a.gamma = d.gamma;
+  a.inv_gm1 = fixed_inv(d.gamma - 1.0);
   a.small_rho = d.small_rho;
   a.small_prs = d.small_prs;
   a.stage = d.stage;

@@ -12,6 +12,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "gp_exact.cuh"
+
 namespace gp {
 
 // variable indices, Src/MHD/mhd.hpp:21-33 and Src/HD/hd.hpp:21-27
@@ -449,6 +451,206 @@ __device__ __forceinline__ void ct_store_ucthlld(const R* ul, const R* ur, const
   c.et = -(aR_1 * vl[VXb] - aL_1 * vr[VXb]) * scrh;
 }
 
+// mhd_prim2cons and the signal speeds with the divisions and roots of `ar`
+// (y = 1/(gamma - 1)); same expressions, so the same values
+template <typename R, typename A>
+__device__ __forceinline__ void mhd_prim2cons(const R* v, R* u, R gmm1, R y, A& ar) {
+  u[RHO] = v[RHO];
+  u[MX1] = v[RHO] * v[VX1];
+  u[MX2] = v[RHO] * v[VX1 + 1];
+  u[MX3] = v[RHO] * v[VX1 + 2];
+  u[BX1] = v[BX1];
+  u[BX2] = v[BX2];
+  u[BX3] = v[BX3];
+  R kinb2 = v[VX1] * v[VX1] + v[VX1 + 1] * v[VX1 + 1] + v[VX1 + 2] * v[VX1 + 2];
+  kinb2 = v[RHO] * kinb2 + v[BX1] * v[BX1] + v[BX2] * v[BX2] + v[BX3] * v[BX3];
+  kinb2 *= R(0.5);
+  u[7] = kinb2 + ar.quot_pos(v[7], gmm1, y);
+}
+
+template <int DIR, typename R, typename A>
+__device__ __forceinline__ void mhd_signal_speed(const R* v, R gamma, R& cmin, R& cmax, A& ar) {
+  constexpr int VXn = VX1 + DIR;
+  const R yr = ar.inv_pos(v[RHO]);
+  const R a2 = ar.quot_pos(gamma * v[7], v[RHO], yr);
+  R b1 = v[BX1 + DIR], b2 = v[BX1 + (DIR + 1) % 3], b3 = v[BX1 + (DIR + 2) % 3];
+  R gpr = a2 * v[RHO];
+  R Btmag2 = b2 * b2 + b3 * b3;
+  R Bmag2 = b1 * b1 + Btmag2;
+  R cf = gpr - Bmag2;
+  cf = gpr + Bmag2 + ar.root(cf * cf + R(4) * gpr * Btmag2);
+  cf = ar.root(ar.quot_pos(R(0.5) * cf, v[RHO], yr));
+  cmax = v[VXn] + cf;
+  cmin = v[VXn] - cf;
+}
+
+// The HLLD solver of mhd_hlld below for faces whose every division and root
+// FastArith covers (ar.bad stays clear; outside the HLL fallback, whose
+// negative star densities set it), in straight-line form: quotients share
+// their divisors' reciprocals, the branch taken by SM, S1L, S1R, Sl and Sr
+// becomes one selection of the side, and the physical flux, the star energy
+// and the double-star state are formed for that side only.  Every value kept
+// is the one mhd_hlld computes.
+template <int DIR, int CT, typename R, typename A>
+__device__ __forceinline__ R mhd_hlld_line(const R* vl, const R* vr, R* flux, R gamma, R ygm,
+                                           R Bn, CTFace<R>& ct, A& ar) {
+  constexpr int VXn = VX1 + DIR, VXt = VX1 + (DIR + 1) % 3, VXb = VX1 + (DIR + 2) % 3;
+  constexpr int MXn = MX1 + DIR, MXt = MX1 + (DIR + 1) % 3, MXb = MX1 + (DIR + 2) % 3;
+  constexpr int BXn = BX1 + DIR, BXt = BX1 + (DIR + 1) % 3, BXb = BX1 + (DIR + 2) % 3;
+  R ul[8], ur[8];
+  const R gmm1 = gamma - R(1);
+  mhd_prim2cons(vl, ul, gmm1, ygm, ar);
+  mhd_prim2cons(vr, ur, gmm1, ygm, ar);
+  R Sl, Sr;
+  {
+    R sl_min, sl_max, sr_min, sr_max;
+    mhd_signal_speed<DIR>(vl, gamma, sl_min, sl_max, ar);
+    mhd_signal_speed<DIR>(vr, gamma, sr_min, sr_max, ar);
+    Sl = GP_MIN(sl_min, sr_min);
+    Sr = GP_MAX(sl_max, sr_max);
+  }
+  const R cmax = GP_MAX(rabs(Sl), rabs(Sr));
+  const R ptl = mhd_ptot(vl), ptr = mhd_ptot(vr);
+  const R dS_1 = ar.inv_pos(Sr - Sl);
+  const R Bx = (Sr * vr[BXn] - Sl * vl[BXn]) * dS_1;
+  const R sBx = (Bx > R(0) ? R(1) : R(-1));
+  const R dul = Sl - vl[VXn], dur = Sr - vr[VXn];
+  const R rdl = ul[RHO] * dul, rdr = ur[RHO] * dur;
+  R scrh = ar.inv_pos(dur * ur[RHO] - dul * ul[RHO]);
+  const R SM = (dur * ur[MXn] - dul * ul[MXn] - ptr + ptl) * scrh;
+  R pts = dur * ur[RHO] * ptl - dul * ul[RHO] * ptr +
+          vl[RHO] * vr[RHO] * dur * dul * (vr[VXn] - vl[VXn]);
+  pts *= scrh;
+  const R dsl = Sl - SM, dsr = Sr - SM;
+  const R ysl = ar.inv(dsl), ysr = ar.inv_pos(dsr);
+  const R rhosl = ar.quot(rdl, dsl, ysl), rhosr = ar.quot_pos(rdr, dsr, ysr);
+  const R sqrL = ar.root(rhosl), sqrR = ar.root(rhosr);
+  const R yqL = ar.inv_pos(sqrL), yqR = ar.inv_pos(sqrR);
+  R S1L = SM - ar.quot(rabs(Bx), sqrL, yqL);
+  R S1R = SM + ar.quot(rabs(Bx), sqrR, yqR);
+
+  if constexpr (CT == CT_UCT_HLLD) {  // ct_store_ucthlld: Sc is SM, the same expression
+    const R Sal = SM - ar.quot(rabs(Bn), sqrL, yqL);
+    const R Sar = SM + ar.quot(rabs(Bn), sqrR, yqR);
+    const R chiL = ar.div((vl[VXn] - SM) * dsl, Sal + Sl - R(2) * SM);
+    const R chiR = ar.div((vr[VXn] - SM) * dsr, Sar + Sr - R(2) * SM);
+    const R nuL = ar.div_pos(Sal + Sl, rabs(Sal) + rabs(Sl));
+    const R nuR = ar.div_pos(Sar + Sr, rabs(Sar) + rabs(Sr));
+    const bool far = rabs(Sar - Sal) > R(1.e-9) * rabs(Sr - Sl);
+    // 0/0 when both vanish, which is not `far`: any divisor will do there
+    const R den = rabs(Sal) + rabs(Sar);
+    const R nuLR = ar.div_pos(Sal + Sar, den > R(0) ? den : R(1));
+    const R dL = R(0.5) * (chiL * nuL - chiL * nuLR) + R(0.5) * (rabs(Sal) - nuLR * Sal);
+    const R dR = R(0.5) * (chiR * nuR - chiR * nuLR) + R(0.5) * (rabs(Sar) - nuLR * Sar);
+    const R aL = R(0.5) * (R(1) + nuLR), aR = R(0.5) * (R(1) - nuLR);
+    ct.dL = far ? dL : R(0.5) * chiL * nuL + R(0.5) * rabs(Sal);
+    ct.dR = far ? dR : R(0.5) * chiR * nuR + R(0.5) * rabs(Sar);
+    ct.aL = far ? aL : R(0.5);
+    ct.aR = far ? aR : R(0.5);
+  }
+  {
+    const R aR_1 = GP_MAX(R(0), Sr), aL_1 = GP_MIN(R(0), Sl);
+    const R y = ar.inv_pos(aR_1 - aL_1);
+    ct.eb = (aR_1 * vl[VXt] - aL_1 * vr[VXt]) * y;
+    ct.et = -(aR_1 * vl[VXb] - aL_1 * vr[VXb]) * y;
+    if constexpr (CT != CT_UCT_HLLD) {
+      ct.aL = aR_1 * y;
+      ct.aR = -aL_1 * y;
+      ct.dR = -aL_1 * aR_1 * y;
+      ct.dL = ct.dR;
+    }
+  }
+
+  // star states: transverse field and velocity of both sides
+  const bool hllc = ((S1L - Sl) < R(1.e-4) * (SM - Sl)) || ((S1R - Sr) > -R(1.e-4) * (Sr - SM));
+  R BtL, BbL, BtR, BbR;
+  {
+    const R kL = ar.div(rdl * dul - Bx * Bx, rdl * dsl - Bx * Bx);
+    const R kR = ar.div(rdr * dur - Bx * Bx, rdr * dsr - Bx * Bx);
+    BtL = ul[BXt] * kL;
+    BbL = ul[BXb] * kL;
+    BtR = ur[BXt] * kR;
+    BbR = ur[BXb] * kR;
+  }
+  if (hllc) {
+    const R flt = vl[BXt] * vl[VXn] - vl[BXn] * vl[VXt];
+    const R frt = vr[BXt] * vr[VXn] - vr[BXn] * vr[VXt];
+    const R flb = vl[BXb] * vl[VXn] - vl[BXn] * vl[VXb];
+    const R frb = vr[BXb] * vr[VXn] - vr[BXn] * vr[VXb];
+    BtL = BtR = (Sr * ur[BXt] - Sl * ul[BXt] + flt - frt) * dS_1;
+    BbL = BbR = (Sr * ur[BXb] - Sl * ul[BXb] + flb - frb) * dS_1;
+    S1L = S1R = SM;
+  }
+  const R wL = ar.div(Bx, rdl), wR = ar.div_pos(Bx, rdr);
+  const R vsL = vl[VXt] - wL * (BtL - ul[BXt]);
+  const R vsR = vr[VXt] - wR * (BtR - ur[BXt]);
+  const R wsL = vl[VXb] - wL * (BbL - ul[BXb]);
+  const R wsR = vr[VXb] - wR * (BbR - ur[BXb]);
+
+  // the side and the region: 0 outside the fan, 1 star, 2 double star
+  const bool outL = Sl >= R(0), outR = !outL && Sr <= R(0);
+  const bool starL = S1L >= R(0), starR = !starL && S1R <= R(0);
+  const bool left = outL || (!outR && (starL || (!starR && SM >= R(0))));
+  const bool outside = outL || outR, twice = !(starL || starR);
+  R v[8], u[8], f[8];
+#pragma unroll
+  for (int nv = 0; nv < 8; nv++) {
+    v[nv] = left ? vl[nv] : vr[nv];
+    u[nv] = (nv >= BX1 && nv <= BX3) ? v[nv] : (left ? ul[nv] : ur[nv]);
+  }
+  u[RHO] = v[RHO];
+  const R S = left ? Sl : Sr, dv = left ? dul : dur, pt = left ? ptl : ptr;
+  const R ds = left ? dsl : dsr, ys = left ? ysl : ysr, rhos = left ? rhosl : rhosr;
+  const R vs = left ? vsL : vsR, ws = left ? wsL : wsR;
+  const R Bt = left ? BtL : BtR, Bb = left ? BbL : BbR;
+  R us[8];
+  us[RHO] = rhos;
+  us[MXn] = rhos * SM;
+  us[MXt] = rhos * vs;
+  us[MXb] = rhos * ws;
+  us[BXn] = Bx;
+  us[BXt] = Bt;
+  us[BXb] = Bb;
+  const R vBs = SM * Bx + vs * Bt + ws * Bb;
+  scrh = v[VXn] * Bx + v[VXt] * u[BXt] + v[VXb] * u[BXb];
+  scrh -= vBs;
+  us[7] = ar.quot(dv * u[7] - pt * v[VXn] + pts * SM + Bx * scrh, ds, ys);
+  R ptf;
+  mhd_flux<DIR>(v, u, f, ptf);
+  // double star: common transverse state
+  {
+    const R dq = sqrL + sqrR, yq = ar.inv_pos(dq);
+    const R vss = ar.quot(sqrL * vsL + sqrR * vsR + (BtR - BtL) * sBx, dq, yq);
+    const R wss = ar.quot(sqrL * wsL + sqrR * wsR + (BbR - BbL) * sBx, dq, yq);
+    const R Btt = ar.quot(sqrL * BtR + sqrR * BtL + sqrL * sqrR * (vsR - vsL) * sBx, dq, yq);
+    const R Bbb = ar.quot(sqrL * BbR + sqrR * BbL + sqrL * sqrR * (wsR - wsL) * sBx, dq, yq);
+    scrh = vBs;
+    scrh -= SM * Bx + vss * Btt + wss * Bbb;
+    const R e = (left ? sqrL : sqrR) * scrh * sBx;
+    const R S1 = left ? S1L : S1R;
+    R uss[8];
+    uss[RHO] = us[RHO];
+    uss[MXn] = us[MXn];
+    uss[MXt] = rhos * vss;
+    uss[MXb] = rhos * wss;
+    uss[BXn] = Bx;
+    uss[BXt] = Btt;
+    uss[BXb] = Bbb;
+    uss[7] = left ? us[7] - e : us[7] + e;
+#pragma unroll
+    for (int nv = 0; nv < 8; nv++) {
+      const R g = f[nv] + S1 * (uss[nv] - us[nv]);
+      f[nv] = outside ? f[nv] : (twice ? g : f[nv]);
+    }
+  }
+#pragma unroll
+  for (int nv = 0; nv < 8; nv++) {
+    const R g = f[nv] + S * (us[nv] - u[nv]);
+    flux[nv] = outside ? f[nv] : g;
+  }
+  return cmax;
+}
+
 // HLLD solver, Src/MHD/hlld.cpp:61-514 (ideal EOS).  vl/vr are the
 // reconstructed primitive states at the interface (normal field already set
 // to the face value).  Returns cmax = max(|Sl|,|Sr|).
@@ -620,6 +822,68 @@ __device__ __forceinline__ R mhd_hlld(const R* vl, const R* vr, R* flux, R gamma
     ct_store_ucthlld<DIR>(ul, ur, vl, vr, Sl, Sr, Bn, ct);
   else
     ct_store_ucthll<DIR>(vl, vr, Sl, Sr, ct);
+  return cmax;
+}
+
+// A face through memory, for the out-of-line solvers: io = vl, vr, gamma, Bn
+// in; flux, face data and cmax out.
+__device__ __forceinline__ void face_in(double* io, const double* vl, const double* vr,
+                                        double gamma, double Bn) {
+#pragma unroll
+  for (int nv = 0; nv < 8; nv++) {
+    io[nv] = vl[nv];
+    io[8 + nv] = vr[nv];
+  }
+  io[16] = gamma;
+  io[17] = Bn;
+}
+__device__ __forceinline__ void face_out(double* io, const double* flux, const CTFace<double>& ct,
+                                         double cmax) {
+#pragma unroll
+  for (int nv = 0; nv < 8; nv++) io[nv] = flux[nv];
+  io[8] = ct.eb;
+  io[9] = ct.et;
+  io[10] = ct.aL;
+  io[11] = ct.aR;
+  io[12] = ct.dL;
+  io[13] = ct.dR;
+  io[14] = cmax;
+}
+__device__ __forceinline__ double face_back(const double* io, double* flux, CTFace<double>& ct) {
+#pragma unroll
+  for (int nv = 0; nv < 8; nv++) flux[nv] = io[nv];
+  ct.eb = io[8];
+  ct.et = io[9];
+  ct.aL = io[10];
+  ct.aR = io[11];
+  ct.dL = io[12];
+  ct.dR = io[13];
+  return io[14];
+}
+
+// mhd_hlld out of line, for the few faces mhd_hlld_line hands back
+template <int DIR, int CT>
+__device__ __noinline__ void mhd_hlld_call(double* io) {
+  double flux[8];
+  CTFace<double> ct;
+  const double cmax = mhd_hlld<DIR, CT>(io, io + 8, flux, io[16], io[17], ct);
+  face_out(io, flux, ct, cmax);
+}
+
+// FP64 HLLD: the straight-line form, and mhd_hlld where its flag is set.
+template <int DIR, int CT>
+__device__ __forceinline__ double mhd_hlld_fp64(const double* vl, const double* vr, double* flux,
+                                                double gamma, double ygm, double Bn,
+                                                CTFace<double>& ct) {
+  FastArith ar;
+  ar.bad = ygm == 0.0;
+  double cmax = mhd_hlld_line<DIR, CT>(vl, vr, flux, gamma, ygm, Bn, ct, ar);
+  if (ar.bad) {
+    double io[18];
+    face_in(io, vl, vr, gamma, Bn);
+    mhd_hlld_call<DIR, CT>(io);
+    cmax = face_back(io, flux, ct);
+  }
   return cmax;
 }
 
@@ -867,6 +1131,88 @@ __device__ __forceinline__ R hd_hllc(const R* vl, const R* vr, R* flux, R gamma)
 #pragma unroll
       for (int nv = 0; nv < 5; nv++) flux[nv] = fR[nv] + Sr * (usr[nv] - ur[nv]);
     }
+  }
+  return cmax;
+}
+
+// hd_hllc for faces FastArith covers, in straight-line form: the side is
+// selected first, and the flux and star state formed for it alone (ygm =
+// 1/(gamma - 1)).  Every value kept is the one hd_hllc computes.
+template <int DIR, typename R, typename A>
+__device__ __forceinline__ R hd_hllc_line(const R* vl, const R* vr, R* flux, R gamma, R ygm,
+                                          A& ar) {
+  constexpr int VXn = VX1 + DIR, VXt = VX1 + (DIR + 1) % 3, VXb = VX1 + (DIR + 2) % 3;
+  constexpr int MXn = MX1 + DIR, MXt = MX1 + (DIR + 1) % 3, MXb = MX1 + (DIR + 2) % 3;
+  const R yl = ar.inv_pos(vl[RHO]), yr = ar.inv_pos(vr[RHO]);
+  const R aL = ar.root(ar.quot_pos(gamma * vl[4], vl[RHO], yl));
+  const R aR = ar.root(ar.quot_pos(gamma * vr[4], vr[RHO], yr));
+  const R sl_min = vl[VXn] - aL, sl_max = vl[VXn] + aL;
+  const R sr_min = vr[VXn] - aR, sr_max = vr[VXn] + aR;
+  const R Sl = GP_MIN(sl_min, sr_min), Sr = GP_MAX(sl_max, sr_max);
+  R vs;
+  {
+    const R qL = vl[4] + vl[RHO] * vl[VXn] * (vl[VXn] - Sl);
+    const R qR = vr[4] + vr[RHO] * vr[VXn] * (vr[VXn] - Sr);
+    const R wL = vl[RHO] * (vl[VXn] - Sl), wR = vr[RHO] * (vr[VXn] - Sr);
+    vs = ar.div(qR - qL, wR - wL);
+  }
+  const bool outL = Sl > R(0), outR = !outL && Sr < R(0);
+  const bool left = outL || (!outR && vs >= R(0));
+  R v[5], u[5], f[5], us[5], p;
+#pragma unroll
+  for (int nv = 0; nv < 5; nv++) v[nv] = left ? vl[nv] : vr[nv];
+  const R S = left ? Sl : Sr, y = left ? yl : yr;
+  u[RHO] = v[RHO];
+  u[MX1] = v[RHO] * v[VX1];
+  u[MX2] = v[RHO] * v[VX1 + 1];
+  u[MX3] = v[RHO] * v[VX1 + 2];
+  R kin = v[VX1] * v[VX1] + v[VX1 + 1] * v[VX1 + 1] + v[VX1 + 2] * v[VX1 + 2];
+  kin = v[RHO] * kin * R(0.5);
+  u[4] = kin + ar.quot_pos(v[4], gamma - R(1), ygm);
+  hd_flux<DIR>(v, u, f, p);
+  const R vx = v[VXn];
+  us[RHO] = ar.div(u[RHO] * (S - vx), S - vs);
+  us[MXn] = us[RHO] * vs;
+  us[MXt] = us[RHO] * v[VXt];
+  us[MXb] = us[RHO] * v[VXb];
+  us[4] = ar.quot(u[4], v[RHO], y) + (vs - vx) * (vs + ar.div(v[4], v[RHO] * (S - vx)));
+  us[4] *= us[RHO];
+#pragma unroll
+  for (int nv = 0; nv < 5; nv++) {
+    const R g = f[nv] + S * (us[nv] - u[nv]);
+    flux[nv] = (outL || outR) ? f[nv] : g;
+  }
+  return GP_MAX(rabs(Sl), rabs(Sr));
+}
+
+// hd_hllc out of line: io = vl, vr, gamma in; flux and cmax out
+template <int DIR>
+__device__ __noinline__ void hd_hllc_call(double* io) {
+  double flux[5];
+  const double cmax = hd_hllc<DIR>(io, io + 5, flux, io[10]);
+#pragma unroll
+  for (int nv = 0; nv < 5; nv++) io[nv] = flux[nv];
+  io[5] = cmax;
+}
+
+template <int DIR>
+__device__ __forceinline__ double hd_hllc_fp64(const double* vl, const double* vr, double* flux,
+                                               double gamma, double ygm) {
+  FastArith ar;
+  ar.bad = ygm == 0.0;
+  double cmax = hd_hllc_line<DIR>(vl, vr, flux, gamma, ygm, ar);
+  if (ar.bad) {
+    double io[11];
+#pragma unroll
+    for (int nv = 0; nv < 5; nv++) {
+      io[nv] = vl[nv];
+      io[5 + nv] = vr[nv];
+    }
+    io[10] = gamma;
+    hd_hllc_call<DIR>(io);
+#pragma unroll
+    for (int nv = 0; nv < 5; nv++) flux[nv] = io[nv];
+    cmax = io[5];
   }
   return cmax;
 }
