@@ -132,10 +132,17 @@ GP_CR_FN double sincos_tab(int j, int k) {
 #endif
 }
 #define GP_CR_TAB_J(j, k) sincos_tab(j, k)
+// round(16 x) for x in [0, 1.125].  Inside the table for any other x too: a NaN
+// (0/0 in the cubic's argument, or a lane whose result is thrown away)
+// converts to INT_MIN.
+GP_CR_FN int table_row(double x) {
+  const int j = (int)(x * 16.0 + 0.5);
+  return j < 0 ? 0 : (j > 18 ? 18 : j);
+}
 
 // double-double sin and cos of x in [0, 1.125]
 GP_CR_FN void sincos_dd(double x, dd& s, dd& c) {
-  const int j = (int)(x * 16.0 + 0.5);
+  const int j = table_row(x);
   const double r = x - (double)j * 0.0625;
   const dd z = two_prod(r, r);
   // sin r = r + r z (-1/3! + z (1/5! + z (-1/7! + z t))),  t = 1/9! - z/11! + z^2/13!
@@ -235,7 +242,7 @@ GP_CR_FN bool round_certain(dd y, double err, double* out) {
 // absolute (j >= 1, sin and cos), 2^-64.2 relative (j = 0, sin).  Returned
 // with the bounds the rounding test uses: 2^-67 absolute, 2^-62 relative.
 GP_CR_FN void sincos_fast(double x, dd& s, dd& c, double& es, double& ec) {
-  const int j = (int)(x * 16.0 + 0.5);
+  const int j = table_row(x);
   const double r = x - (double)j * 0.0625;
   const dd z = two_prod(r, r);
   const double zh = z.hi;
@@ -290,7 +297,7 @@ GP_CR_FN void sincos_fast(double x, dd& s, dd& c, double& es, double& ec) {
 // precision only: the Newton step of acos_cr divides by it, where relative
 // accuracy 2^-50 is ample.
 GP_CR_FN void sin_fast_cos_d(double x, dd& s, double& es, double& cd) {
-  const int j = (int)(x * 16.0 + 0.5);
+  const int j = table_row(x);
   const double r = x - (double)j * 0.0625;
   const dd z = two_prod(r, r);
   const double zh = z.hi;

@@ -94,3 +94,11 @@ def test_fast_path_decides_nearly_every_call(crm):
     crm(1, theta)                               # sin and cos share one slow call
     slow = crm.slow_calls() - before
     assert slow < 0.005 * 2 * x.size, slow
+
+
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_nan_stays_inside_the_table(crm, which):
+    """A NaN argument (0/0 in the cubic, or a lane whose result is thrown away)
+    gives NaN: its table row is clamped, not the integer a NaN converts to."""
+    ours, _ = crm(which, np.array([np.nan, -np.nan]))
+    assert np.isnan(ours).all()
