@@ -330,7 +330,6 @@ struct gp_handle {
   cudaStream_t stream;
   bool mixed;
   gp::SchemeKey key;
-  int seg;
   // device state
   double* U[2];
   double* V;
@@ -494,8 +493,8 @@ int enqueue_step(gp_handle* h, double* hist, int slot, cudaEvent_t* ev = nullptr
   auto launch = [&](const gp::StageDesc& sd) {
     gp::GridDims g = grid_dims(h);
     cudaEvent_t* e = ev ? ev + (sd.stage - 1) * 2 * per_stage : nullptr;
-    return h->mixed ? gp::launch_stage_mixed(sd, g, h->key, h->seg, h->stream, e)
-                    : gp::launch_stage_fp64(sd, g, h->key, h->seg, h->stream, e);
+    return h->mixed ? gp::launch_stage_mixed(sd, g, h->key, h->stream, e)
+                    : gp::launch_stage_fp64(sd, g, h->key, h->stream, e);
   };
   // stage 1: (U^n, B^n) -> (U1, B1)
   if (h->padded) {
@@ -766,37 +765,6 @@ int gp_create(const gp_grid_desc* grid, const gp_scheme* scheme, void* stream,
                          : scheme->reconstruction == GP_REC_LIMO3   ? 10  /* LIM_LIMO3 */
                          : scheme->reconstruction == GP_REC_WENO3   ? 11  /* LIM_WENO3 */
                                                                     : scheme->limiter};
-  // pencil segment for the marching sweeps: enough threads to fill 148 SMs,
-  // then, among that length and its halves down to a quarter, the one whose
-  // y and z sweeps take the fewest (waves of resident blocks) x (cells a
-  // block marches, + 2 for its start-up): a last wave that fills few SMs
-  // costs a whole wave.  At 256^3 the FP64 sweeps (4 blocks per SM) take
-  // 32 (y/z 1.33 -> 1.29 ms against 64), the mixed ones (5 per SM) keep 64.
-  {
-    long long cols = (long long)h->px * (h->ndim == 3 ? h->pz : 1);
-    int nd = h->py;
-    int seg = 64;
-    while (seg > 4 && cols * ((nd + seg - 1) / seg) < 148LL * 1024) seg /= 2;
-    const long long resident =
-        148LL * gp::sweep_m_blocks_per_sm(scheme->physics, h->mixed);
-    // blocks of SWEEP_THREADS (128) columns, x and transverse taken together
-    const long long cy = ((long long)h->px * (h->ndim == 3 ? h->pz : 1) + 127) / 128;
-    const long long cz = ((long long)h->px * h->py + 127) / 128;
-    auto cost = [&](int S) {
-      long long c = 0;
-      const long long by = cy * ((h->py + S - 1) / S);
-      c += (by + resident - 1) / resident * (S + 2);
-      if (h->ndim == 3) {
-        const long long bz = cz * ((h->pz + S - 1) / S);
-        c += (bz + resident - 1) / resident * (S + 2);
-      }
-      return c;
-    };
-    int best = seg;
-    for (int S = seg / 2; S >= 4 && S >= seg / 4; S /= 2)
-      if (cost(S) < cost(best)) best = S;
-    h->seg = best;
-  }
   const size_t cell = sizeof(double) * h->pn;
   const size_t ctb = (h->mixed ? sizeof(float) : sizeof(double)) * h->pn;
   bool ok = true;

@@ -573,7 +573,7 @@ int gp_batch_add(gp_batch* b, const gp_grid_desc* grid, const gp_scheme* scheme,
       }
       a.dtdx = sc->dtdx;
       a.gamma = scheme->gamma;
-      a.inv_gm1 = gp::fixed_inv(scheme->gamma - 1.0);
+      a.inv_gm1 = gp::gamma_inv(scheme->gamma);
       a.small_rho = scheme->small_rho;
       a.small_prs = scheme->small_prs;
       a.stage = stage;

@@ -99,7 +99,9 @@ __device__ void batch_cell_tile_mixed(const BatchSlot& s, const BatchTile& t, in
 
 // Shared memory a block needs (largest staging area of any phase).
 constexpr int batch_smem_bytes() {
-  return (int)sizeof(double) * sweep_x_stage_doubles<8>();
+  return (int)sizeof(double) * (sweep_x_stage_doubles<8>() > sweep_m_stage_doubles<8>()
+                                    ? sweep_x_stage_doubles<8>()
+                                    : sweep_m_stage_doubles<8>());
 }
 
 }  // namespace gp

@@ -63,8 +63,8 @@ template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM>
 __device__ __noinline__ void tile_sweep_x(const StageArgs<CTT>& a, Grid3 g, int idx,
                                           double* smem) {
   const int tid = threadIdx.x;
-  sweep_x_row<PHYS, NV, NDIM, RS, CT, LIM, RT, CTT>(a, g, idx * BATCH_ROWS_PER_TILE + (tid >> 5),
-                                                    smem, tid);
+  sweep_x_row<PHYS, NV, NDIM, RS, CT, LIM, RT, CTT>(a, g, idx * BATCH_ROWS_PER_TILE + (tid >> 5), 0,
+                                                    g.nx, smem, tid);
 }
 
 template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR>

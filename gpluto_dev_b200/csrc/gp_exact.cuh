@@ -43,7 +43,6 @@ struct PlainArith {
   __device__ __forceinline__ R quot(R a, R b, R) { return a / b; }
   __device__ __forceinline__ R quot_pos(R a, R b, R) { return a / b; }
   __device__ __forceinline__ R div(R a, R b) { return a / b; }
-  __device__ __forceinline__ R div_pos(R a, R b) { return a / b; }
   __device__ __forceinline__ R root(R a) { return sqrt(a); }
   __device__ __forceinline__ R root0(R a) { return sqrt(a); }
 };
@@ -62,6 +61,10 @@ struct FastArith {
   // RN(1/b), b > 0 (a negative b sets the flag)
   __device__ __forceinline__ double inv_pos(double b) {
     bad |= (unsigned)__double2hiint(b) - kDivLo > kDivSpan;
+    return inv_in(b);
+  }
+  // the same without the test, for a divisor the caller's bounds cover
+  __device__ __forceinline__ double inv_in(double b) {
     double y0;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(b));
     const double e = __fma_rn(-b, y0, 1.0);
@@ -92,7 +95,28 @@ struct FastArith {
     return __fma_rn(__fma_rn(-b, q, a), y, q);
   }
   __device__ __forceinline__ double div(double a, double b) { return quot(a, b, inv(b)); }
-  __device__ __forceinline__ double div_pos(double a, double b) { return quot(a, b, inv_pos(b)); }
+  // A dividend used with quot_bpos: 0 or in [2^-700, 2^700]
+  __device__ __forceinline__ void check(double a) {
+    const unsigned lo = (unsigned)__double2loint(a);
+    const unsigned k = ((unsigned)__double2hiint(a) & 0x7fffffffu) | (lo < 1u ? lo : 1u);
+    bad |= (k - kNumLo > kNumSpan) & (k != 0u);
+  }
+  // RN(a/b), b > 0, for a dividend that check() or the caller's bounds cover.
+  // The remainder is rounded downwards, which leaves the quotient's rounding
+  // as it is (checked exhaustively for 4 to 12 bits) and gives a zero
+  // dividend the remainder -0, so that a zero quotient keeps its sign.
+  __device__ __forceinline__ double quot_bpos(double a, double b, double y) {
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rd(-b, q, a), y, q);
+  }
+  // RN(a/b), both checked, b of either sign
+  __device__ __forceinline__ double div_any(double a, double b) {
+    check(a);
+    const int hi = __double2hiint(b), s = hi & (int)0x80000000;
+    const double m = __hiloint2double(hi & 0x7fffffff, __double2loint(b));
+    const double t = __hiloint2double(__double2hiint(a) ^ s, __double2loint(a));
+    return quot_bpos(t, m, inv_pos(m));
+  }
   // RN(sqrt(a)), a > 0
   __device__ __forceinline__ double root(double a) {
     bad |= (unsigned)__double2hiint(a) - kRootLo > kRootSpan;
@@ -103,12 +127,30 @@ struct FastArith {
     const double g = __dmul_rn(a, y1);
     return __fma_rn(__fma_rn(-g, g, a), __dmul_rn(0.5, y1), g);
   }
+  // star densities: root() marks the negative ones
+  __device__ __forceinline__ void densities(double, double) {}
   // root of a >= +0
   __device__ __forceinline__ double root0(double a) {
     const bool zero = __double_as_longlong(a) == 0;
     const double r = root(zero ? 1.0 : a);
     return zero ? a : r;
   }
+};
+
+// FP32 of the mixed form: one approximate reciprocal per divisor (the units
+// compile with approximate division, so a quotient is such a product there
+// too).  `bad` only marks negative star densities (the HLL fallback).
+struct FloatArith {
+  static constexpr bool FAST = true;
+  bool bad = false;
+  __device__ __forceinline__ float inv_pos(float b) { return 1.0f / b; }
+  __device__ __forceinline__ float inv_in(float b) { return 1.0f / b; }
+  __device__ __forceinline__ void check(float) {}
+  __device__ __forceinline__ float quot_pos(float a, float, float y) { return a * y; }
+  __device__ __forceinline__ float quot_bpos(float a, float, float y) { return a * y; }
+  __device__ __forceinline__ float div_any(float a, float b) { return a / b; }
+  __device__ __forceinline__ float root(float a) { return sqrtf(a); }
+  __device__ __forceinline__ void densities(float l, float r) { bad = l < 0.0f || r < 0.0f; }
 };
 
 // RN(a/b) for a divisor fixed over a launch, y = RN(1/b) formed once; the
@@ -125,6 +167,13 @@ __device__ __forceinline__ float fixed_quot(float a, float b, float) { return a 
 __host__ __device__ inline double fixed_inv(double b) {
   const double m = b < 0 ? -b : b;
   return (m >= 0x1p-200 && m <= 0x1p200) ? 1.0 / b : 0.0;
+}
+// 1/(gamma - 1) for the solvers, 0 (the operators) for a gamma out of
+// [1 + 2^-40, 2^40]: a pressure whose gamma p passed its test is then a
+// dividend that needs none
+__host__ __device__ inline double gamma_inv(double gamma) {
+  const double b = gamma - 1.0;
+  return (b >= 0x1p-40 && gamma <= 0x1p40) ? 1.0 / b : 0.0;
 }
 
 }  // namespace gp

@@ -131,7 +131,7 @@ constexpr int sweep_x_minb() {
 }
 template <int PHYS, typename R>
 constexpr int sweep_m_minb() {
-  return PHYS == PHYS_RMHD ? 3 : (sizeof(R) == 4 ? 5 : 4);
+  return PHYS == PHYS_RMHD ? (sizeof(R) == 4 ? 3 : 2) : (sizeof(R) == 4 ? 5 : 4);
 }
 
 // whether conserved component nv receives a flux difference that survives
@@ -148,9 +148,8 @@ __device__ __forceinline__ R riemann(const R* vl, const R* vr, R* flux, R gamma,
                                      CTFace<R>& ct, uint32_t& err) {
   if constexpr (PHYS == PHYS_MHD) {
     R cm;
-    if constexpr (RS == RS_HLLD && sizeof(R) == sizeof(double))
-      cm = mhd_hlld_fp64<DIR, CT>(vl, vr, flux, gamma, ygm, Bn, ct);
-    else if constexpr (RS == RS_HLLD) cm = mhd_hlld<DIR, CT>(vl, vr, flux, gamma, Bn, ct);
+    if constexpr (RS == RS_HLLD)
+      cm = mhd_hlld_face<DIR, CT>(vl, vr, flux, gamma, ygm, Bn, ct);
     else if constexpr (RS == RS_TVDLF) cm = mhd_tvdlf<DIR>(vl, vr, flux, gamma, ct);
     else if constexpr (RS == RS_HLLC) cm = mhd_hllc<DIR>(vl, vr, flux, gamma, ct);
     else cm = mhd_hll<DIR>(vl, vr, flux, gamma, ct);
@@ -250,15 +249,31 @@ __device__ __forceinline__ void store_ct(const StageArgs<CTT>& a, int dir, long 
 // Face f (between cells f-1 and f) is computed by lane f%32; the lane then
 // updates cell f-1.  The first face's flux is kept for cell nx-1.
 // ---------------------------------------------------------------------
-// Staging area of one 128-thread block: [2 buffers][SL values][128 threads]
-// (+ [2 buffers][4 warps][NV] for the second-next cell with PPM).
+// Staging area of one 128-thread block, in doubles.  x-sweep (PLM, LimO3,
+// WENO3): per warp the layout of XRow; PPM, MP5 and WENO-Z: [2 buffers][SL
+// values][128 threads] and [2 buffers][4 warps][NV] for the second-next cell.
+template <int NV>
+struct XRow {
+  static constexpr int CELLS = 34;                   // cells c0-1 .. c0+32 of a chunk
+  static constexpr int V = 0;                        // [2][NV][CELLS]
+  static constexpr int B = V + 2 * NV * CELLS;       // [2][32] face fields
+  static constexpr int E = B + 64;                   // [NV][33] right edge values
+  static constexpr int F = E + NV * 33;              // [NV + 1][33] fluxes, signal speed
+  static constexpr int F0 = F + (NV + 1) * 33;       // [NV + 1] those of the row's first face
+  static constexpr int SIZE = F0 + NV + 1;
+};
 template <int NV, int LIM = LIM_MC>
 constexpr int sweep_x_stage_doubles() {
-  return 2 * (2 * NV + 1) * SWEEP_THREADS +
-         ((LIM == LIM_PPM || five_point<LIM>()) ? 2 * (SWEEP_THREADS / 32) * NV : 0);
+  return (LIM == LIM_PPM || five_point<LIM>())
+             ? 2 * (2 * NV + 1) * SWEEP_THREADS + 2 * (SWEEP_THREADS / 32) * NV
+             : XRow<NV>::SIZE * (SWEEP_THREADS / 32);
 }
-template <int NV>
-constexpr int sweep_m_stage_doubles() { return 2 * (NV + 1) * SWEEP_THREADS; }
+// y/z sweeps: a ring of four cells and two face fields per thread (PLM,
+// LimO3, WENO3), two cells and face fields otherwise
+template <int NV, int LIM = LIM_MC>
+constexpr int sweep_m_stage_doubles() {
+  return ((LIM == LIM_PPM || five_point<LIM>()) ? 2 * (NV + 1) : 4 * NV + 2) * SWEEP_THREADS;
+}
 
 // Piecewise parabolic x-row (one warp per row).  Lane l of a chunk owns
 // cell/face f = c0 + l: it forms the constrained value of face f from cells
@@ -596,12 +611,48 @@ __device__ __forceinline__ void sweep_x_row_mp5(const StageArgs<CTT>& a, const G
   if (err) atomicOr(a.err, err);
 }
 
-// One x-row per warp.  `stg_` is the block's staging area
-// (sweep_x_stage_doubles<NV>() doubles of shared memory), `tid` the thread's
-// index in its 128-thread block.
+// PLM, LimO3 or WENO3 edge values of cell v0 between vm and vp: left (vR,
+// the right state of its left face) and right (vLn, the left state of its
+// right face).
+template <int PHYS, int NV, int LIM, typename R>
+__device__ __forceinline__ void cell_edges(const R* vm, const R* v0, const R* vp, R dx, R* vR,
+                                           R* vLn) {
+  if constexpr (three_point<LIM>()) {
+#pragma unroll
+    for (int nv = 0; nv < NV; nv++) {
+      vR[nv] = edge3<LIM>(vp[nv], v0[nv], vm[nv], dx);
+      vLn[nv] = edge3<LIM>(vm[nv], v0[nv], vp[nv], dx);
+    }
+    const R qm[2] = {vm[RHO], vm[NV - 1]}, qp[2] = {vp[RHO], vp[NV - 1]};
+    mp5_fallback<PHYS, NV>(v0, qm, qp, vR, vLn);
+  } else {
+#pragma unroll
+    for (int nv = 0; nv < NV; nv++) {
+      const R dv = half_limit<LIM>(vp[nv] - v0[nv], v0[nv] - vm[nv]);
+      vR[nv] = v0[nv] - dv;
+      vLn[nv] = v0[nv] + dv;
+    }
+    if constexpr (PHYS == PHYS_RMHD) rmhd_vel_limit<NV>(v0, vR, vLn);
+  }
+}
+
+// The cells [s0, s1) of one x-row by one warp.  Chunks of 32 faces: lane l
+// solves face f = c0 + l and updates cell f-1.  Cells (with a halo of one on
+// each side), right edge values and fluxes pass between the lanes and from
+// chunk to chunk through the warp's shared memory (XRow), so that nothing but
+// the face's own two states is live in registers across the Riemann solver:
+// with shuffles and a carry in every lane the FP64 kernel spilled 212 bytes a
+// thread at 168 registers, and the spills' write-through traffic was twice
+// the kernel's own (34.5 M sectors against 12.3 M at 160^3).  256^3, with the
+// straight-line HLLD: 1308 -> 1000 us.
+// A whole periodic row solves faces 0 .. nx-1 and keeps face 0 for its last
+// cell; a part of a row (s0 > 0 or s1 < nx, used when whole rows would leave
+// SMs idle) or a row with an outflow high side also solves face s1.
+// `stg_` is the block's staging area (sweep_x_stage_doubles<NV, LIM>()
+// doubles of shared memory), `tid` the thread's index in its 128-thread block.
 template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, typename R, typename CTT>
 __device__ __forceinline__ void sweep_x_row(const StageArgs<CTT>& a, const Grid3& g, int row,
-                                            double* stg_, int tid) {
+                                            int s0, int s1, double* stg_, int tid) {
   if constexpr (LIM == LIM_PPM) {
     sweep_x_row_ppm<PHYS, NV, NDIM, RS, CT, R, CTT>(a, g, row, stg_, tid);
     return;
@@ -610,119 +661,103 @@ __device__ __forceinline__ void sweep_x_row(const StageArgs<CTT>& a, const Grid3
     sweep_x_row_mp5<PHYS, NV, NDIM, RS, CT, LIM, R, CTT>(a, g, row, stg_, tid);
     return;
   }
-  constexpr unsigned FULL = 0xffffffffu;
-  constexpr int SL = 2 * NV + 1;  // staged doubles per lane: V[f], V[f+1], Bs[f]
-  double(*stg)[SL][SWEEP_THREADS] = reinterpret_cast<double(*)[SL][SWEEP_THREADS]>(stg_);
+  using L = XRow<NV>;
   const int lane = tid & 31;
-  if (row >= g.ny * g.nz) return;  // warp-uniform
+  if (row >= g.ny * g.nz || s0 >= s1) return;  // warp-uniform
   const int nx = g.nx;
   const unsigned ob = g.outflow;
-  // faces solved: nx (periodic: face nx is face 0) or nx+1 (outflow high side)
-  const int nf = nx + (int)((ob >> 1) & 1u);
+  const bool whole = s0 == 0 && s1 == nx && !((ob >> 1) & 1u);
+  const int f1 = whole ? nx : s1 + 1;  // one past the last face solved
   const long long n = g.n;
   const long long rb = (long long)row * nx;
   const R gamma = (R)a.gamma;
+  double* sv = stg_ + (tid >> 5) * L::SIZE;
+  double* sb = sv + L::B;
+  R* se = reinterpret_cast<R*>(sv + L::E);
+  R* sf = reinterpret_cast<R*>(sv + L::F);
+  R* sf0 = reinterpret_cast<R*>(sv + L::F0);
 
-  // carried state of cell c0-1 (uniform over lanes)
-  R pV[NV], pVLn[NV], pF[NV], pCm = R(0);
-  {
-    R vm[NV], v0[NV], vp[NV];
-    load_cell<NV>(a.V, n, rb + gidx(-2, nx, ob, 0), vm);
-    load_cell<NV>(a.V, n, rb + gidx(-1, nx, ob, 0), v0);
-    load_cell<NV>(a.V, n, rb + 0, vp);
-    R pVR[NV];
-    if constexpr (three_point<LIM>()) {
-      const R dx = (R)a.dx[0];
-#pragma unroll
-      for (int nv = 0; nv < NV; nv++) {
-        pV[nv] = v0[nv];
-        pVLn[nv] = edge3<LIM>(vm[nv], v0[nv], vp[nv], dx);
-        pVR[nv] = edge3<LIM>(vp[nv], v0[nv], vm[nv], dx);
-        pF[nv] = R(0);
-      }
-      const R qm[2] = {vm[RHO], vm[NV - 1]}, qp[2] = {vp[RHO], vp[NV - 1]};
-      mp5_fallback<PHYS, NV>(v0, qm, qp, pVR, pVLn);
-    } else {
-#pragma unroll
-      for (int nv = 0; nv < NV; nv++) {
-        R dv = limit<LIM>(vp[nv] - v0[nv], v0[nv] - vm[nv]);
-        pV[nv] = v0[nv];
-        pVLn[nv] = v0[nv] + R(0.5) * dv;
-        pVR[nv] = v0[nv] - R(0.5) * dv;
-        pF[nv] = R(0);
-      }
-      if constexpr (PHYS == PHYS_RMHD) rmhd_vel_limit<NV>(v0, pVR, pVLn);
-    }
-  }
-  R fF[NV], fCm = R(0);  // flux of face 0 (lane 0 of the first chunk)
-  R F[NV], cm = R(0);
-#pragma unroll
-  for (int nv = 0; nv < NV; nv++) { fF[nv] = R(0); F[nv] = R(0); }
-  uint32_t err = 0;
-
-  // stage chunk c0 into buffer b: V[f], V[f+1] (lanes that cannot take it
-  // from the next lane), Bs[f]
+  // cells c0-1 .. c0+32 and faces c0 .. c0+31 into buffer b
   auto stage_chunk = [&](int c0, int b) {
-    const int f = c0 + lane;
-    const int fc = f < nx ? f : nx - 1;
+    const int cl = gidx(min(c0 - 1 + lane, s1 + 1), nx, ob, 0);
+    double* d = sv + b * (NV * L::CELLS) + lane;
 #pragma unroll
-    for (int nv = 0; nv < NV; nv++) cp_async8(&stg[b][nv][tid], a.V + nv * n + rb + fc);
-    if (lane == 31 || f + 1 >= nf) {
-      const int fp = gidx(fc + 1, nx, ob, 0);
+    for (int nv = 0; nv < NV; nv++) cp_async8(d + nv * L::CELLS, a.V + nv * n + rb + cl);
+    if (lane < 2) {
+      const int ch = gidx(min(c0 + 31 + lane, s1 + 1), nx, ob, 0);
 #pragma unroll
-      for (int nv = 0; nv < NV; nv++) cp_async8(&stg[b][NV + nv][tid], a.V + nv * n + rb + fp);
+      for (int nv = 0; nv < NV; nv++) cp_async8(d + nv * L::CELLS + 32, a.V + nv * n + rb + ch);
     }
-    if constexpr (PHYS != PHYS_HD) cp_async8(&stg[b][2 * NV][tid], a.Bs[0] + rb + fc);
+    if constexpr (PHYS != PHYS_HD)
+      cp_async8(sb + b * 32 + lane, a.Bs[0] + rb + gidx(min(c0 + lane, s1), nx, ob, 0));
     cp_async_commit();
   };
-  stage_chunk(0, 0);
+  stage_chunk(s0, 0);
+  {  // right edge of cell s0-1: the left state of the first face
+    R vm[NV], v0[NV], vp[NV], e[NV], w[NV];
+    load_cell<NV>(a.V, n, rb + gidx(s0 - 2, nx, ob, 0), vm);
+    load_cell<NV>(a.V, n, rb + gidx(s0 - 1, nx, ob, 0), v0);
+    load_cell<NV>(a.V, n, rb + s0, vp);
+    cell_edges<PHYS, NV, LIM>(vm, v0, vp, (R)a.dx[0], w, e);
+    __syncwarp();  // an earlier row's reads of the exchange areas are done
+    if (lane == 0) {
+#pragma unroll
+      for (int nv = 0; nv < NV; nv++) se[nv * 33] = e[nv];
+    }
+  }
+  R F[NV], cm = R(0);
+#pragma unroll
+  for (int nv = 0; nv < NV; nv++) F[nv] = R(0);
+  uint32_t err = 0;
   int buf = 0;
-  for (int c0 = 0; c0 < nf; c0 += 32, buf ^= 1) {
+  for (int c0 = s0; c0 < f1; c0 += 32, buf ^= 1) {
     const int f = c0 + lane;
-    const bool act = f < nf;
-    stage_chunk(c0 + 32 < nf ? c0 + 32 : c0, buf ^ 1);   // prefetch the next chunk
+    const bool act = f < f1;
+    stage_chunk(c0 + 32 < f1 ? c0 + 32 : c0, buf ^ 1);   // prefetch the next chunk
     cp_async_wait1();
-    R Vc[NV], Vm1[NV], Vp1[NV], vL[NV], vR[NV], vLn[NV];
-    const bool selfp1 = (lane == 31) || (f + 1 >= nf);
+    __syncwarp();
+    R vL[NV], vR[NV];
+    {
+      R vm[NV], v0[NV], vp[NV], e[NV];
+      const double* d = sv + buf * (NV * L::CELLS) + lane;
+      if constexpr (sizeof(R) == 8) {
 #pragma unroll
-    for (int nv = 0; nv < NV; nv++) {
-      Vc[nv] = (R)stg[buf][nv][tid];
-      if (selfp1) Vp1[nv] = (R)stg[buf][NV + nv][tid];
-    }
-    if constexpr (three_point<LIM>()) {
-      const R dx = (R)a.dx[0];
+        for (int nv = 0; nv < NV; nv++) {
+          vm[nv] = d[nv * L::CELLS];
+          v0[nv] = d[nv * L::CELLS + 1];
+          vp[nv] = d[nv * L::CELLS + 2];
+        }
+      } else {  // FP32: each cell is converted once, by its own lane, and shuffled
+        R h[NV];
 #pragma unroll
-      for (int nv = 0; nv < NV; nv++) {
-        R up = __shfl_up_sync(FULL, Vc[nv], 1);
-        R dn = __shfl_down_sync(FULL, Vc[nv], 1);
-        Vm1[nv] = (lane == 0) ? pV[nv] : up;
-        if (!selfp1) Vp1[nv] = dn;
-        vR[nv] = edge3<LIM>(Vp1[nv], Vc[nv], Vm1[nv], dx);
-        vLn[nv] = edge3<LIM>(Vm1[nv], Vc[nv], Vp1[nv], dx);
+        for (int nv = 0; nv < NV; nv++) v0[nv] = (R)d[nv * L::CELLS + 1];
+        if (lane == 0 || lane == 31) {
+#pragma unroll
+          for (int nv = 0; nv < NV; nv++) h[nv] = (R)d[nv * L::CELLS + (lane == 0 ? 0 : 2)];
+        }
+#pragma unroll
+        for (int nv = 0; nv < NV; nv++) {
+          const R up = __shfl_up_sync(0xffffffffu, v0[nv], 1);
+          const R dn = __shfl_down_sync(0xffffffffu, v0[nv], 1);
+          vm[nv] = lane == 0 ? h[nv] : up;
+          vp[nv] = lane == 31 ? h[nv] : dn;
+        }
       }
-      const R qm[2] = {Vm1[RHO], Vm1[NV - 1]}, qp[2] = {Vp1[RHO], Vp1[NV - 1]};
-      mp5_fallback<PHYS, NV>(Vc, qm, qp, vR, vLn);
-    } else {
+      cell_edges<PHYS, NV, LIM>(vm, v0, vp, (R)a.dx[0], vR, e);
 #pragma unroll
-      for (int nv = 0; nv < NV; nv++) {
-        R up = __shfl_up_sync(FULL, Vc[nv], 1);
-        R dn = __shfl_down_sync(FULL, Vc[nv], 1);
-        Vm1[nv] = (lane == 0) ? pV[nv] : up;
-        if (!selfp1) Vp1[nv] = dn;
-        R dv = limit<LIM>(Vp1[nv] - Vc[nv], Vc[nv] - Vm1[nv]);
-        vR[nv] = Vc[nv] - R(0.5) * dv;
-        vLn[nv] = Vc[nv] + R(0.5) * dv;
+      for (int nv = 0; nv < NV; nv++) se[nv * 33 + lane + 1] = e[nv];
+      __syncwarp();
+#pragma unroll
+      for (int nv = 0; nv < NV; nv++) vL[nv] = se[nv * 33 + lane];
+      __syncwarp();
+      if (lane == 31) {
+#pragma unroll
+        for (int nv = 0; nv < NV; nv++) se[nv * 33] = e[nv];
       }
-      if constexpr (PHYS == PHYS_RMHD) rmhd_vel_limit<NV>(Vc, vR, vLn);
-    }
-#pragma unroll
-    for (int nv = 0; nv < NV; nv++) {
-      R l = __shfl_up_sync(FULL, vLn[nv], 1);
-      vL[nv] = (lane == 0) ? pVLn[nv] : l;
     }
     R Bn = R(0);
     if constexpr (PHYS != PHYS_HD) {
-      Bn = (R)stg[buf][2 * NV][tid];  // Src/States/plm_states.cpp:184-189
+      Bn = (R)sb[buf * 32 + lane];  // Src/States/plm_states.cpp:184-189
       vL[BX1] = Bn;
       vR[BX1] = Bn;
     }
@@ -732,57 +767,57 @@ __device__ __forceinline__ void sweep_x_row(const StageArgs<CTT>& a, const Grid3
 #pragma unroll
     for (int nv = 0; nv < NV; nv++)
       if (act && rhs_var<PHYS, NDIM>(nv) && isnan(F[nv])) fe |= ERR_NAN | ERR_QUIT;
-    if (fe && face_counts(g, 0, f, 1, row % g.ny, 2, row / g.ny)) err |= fe;
+    if (act && fe && face_counts(g, 0, f, 1, row % g.ny, 2, row / g.ny)) err |= fe;
     if constexpr (PHYS != PHYS_HD) {
-      if (act) store_ct<CT>(a, 0, rb + f, ct);
+      if (act && f < s1) store_ct<CT>(a, 0, rb + f, ct);
     }
     // flux of face f-1 and cell update of cell f-1
-    R Fm1[NV];
 #pragma unroll
-    for (int nv = 0; nv < NV; nv++) {
-      R t = __shfl_up_sync(FULL, F[nv], 1);
-      Fm1[nv] = (lane == 0) ? pF[nv] : t;
-    }
-    R cmm1;
-    {
-      R t = __shfl_up_sync(FULL, cm, 1);
-      cmm1 = (lane == 0) ? pCm : t;
-    }
-    if (act && f >= 1)
-      cell_update<PHYS, NV, NDIM>(a, n, rb + (f - 1), Fm1, F, cmm1, cm, 0);
-    if (c0 == 0) {
+    for (int nv = 0; nv < NV; nv++)
+      if (rhs_var<PHYS, NDIM>(nv)) sf[nv * 33 + lane + 1] = F[nv];
+    sf[NV * 33 + lane + 1] = cm;
+    if (c0 == s0 && lane == 0) {
 #pragma unroll
-      for (int nv = 0; nv < NV; nv++) fF[nv] = F[nv];
-      fCm = cm;
+      for (int nv = 0; nv < NV; nv++) sf0[nv] = F[nv];
+      sf0[NV] = cm;
     }
+    __syncwarp();
+    if (act && f > s0) {
+      R Fm1[NV];
 #pragma unroll
-    for (int nv = 0; nv < NV; nv++) {
-      pV[nv] = __shfl_sync(FULL, Vc[nv], 31);
-      pVLn[nv] = __shfl_sync(FULL, vLn[nv], 31);
-      pF[nv] = __shfl_sync(FULL, F[nv], 31);
+      for (int nv = 0; nv < NV; nv++)
+        if (rhs_var<PHYS, NDIM>(nv)) Fm1[nv] = sf[nv * 33 + lane];
+      cell_update<PHYS, NV, NDIM>(a, n, rb + (f - 1), Fm1, F, sf[NV * 33 + lane], cm, 0);
     }
-    pCm = __shfl_sync(FULL, cm, 31);
+    __syncwarp();
+    if (lane == 31) {
+#pragma unroll
+      for (int nv = 0; nv < NV; nv++)
+        if (rhs_var<PHYS, NDIM>(nv)) sf[nv * 33] = F[nv];
+      sf[NV * 33] = cm;
+    }
   }
   cp_async_wait0();
-  // periodic: cell nx-1 uses F[nx-1] (lane (nx-1)%32 of the last chunk) and
-  // F[nx] = F[0]; with an outflow high side face nx was solved in the loop
-  if (nf == nx) {
+  // cell nx-1 of a whole periodic row: F[nx-1] (lane (nx-1)%32 of the last
+  // chunk) and F[nx] = F[0]
+  if (whole && lane == ((nx - 1) & 31)) {
     R F0[NV];
 #pragma unroll
-    for (int nv = 0; nv < NV; nv++) F0[nv] = __shfl_sync(FULL, fF[nv], 0);
-    R cm0 = __shfl_sync(FULL, fCm, 0);
-    if (lane == ((nx - 1) & 31))
-      cell_update<PHYS, NV, NDIM>(a, n, rb + (nx - 1), F, F0, cm, cm0, 0);
+    for (int nv = 0; nv < NV; nv++) F0[nv] = sf0[nv];
+    cell_update<PHYS, NV, NDIM>(a, n, rb + (nx - 1), F, F0, cm, sf0[NV], 0);
   }
   if (err) atomicOr(a.err, err);
 }
 
 template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, typename R, typename CTT>
 __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_x_minb<PHYS, R>()))
-    sweep_x_kernel(StageArgs<CTT> a, Grid3 g) {
+    sweep_x_kernel(StageArgs<CTT> a, Grid3 g, int nseg) {
   __shared__ double stg[sweep_x_stage_doubles<NV, LIM>()];
-  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  sweep_x_row<PHYS, NV, NDIM, RS, CT, LIM, R, CTT>(a, g, row, stg, threadIdx.x);
+  const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int row = w / nseg, q = w - row * nseg;
+  sweep_x_row<PHYS, NV, NDIM, RS, CT, LIM, R, CTT>(a, g, row, (int)((long long)g.nx * q / nseg),
+                                                   (int)((long long)g.nx * (q + 1) / nseg), stg,
+                                                   threadIdx.x);
 }
 
 // ---------------------------------------------------------------------
@@ -998,7 +1033,14 @@ __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3
     sweep_m_col_mp5<PHYS, NV, NDIM, RS, CT, LIM, DIR, R, CTT>(a, g, i, t, seg, S, stg_, tid);
     return;
   }
-  double(*stg)[NV + 1][SWEEP_THREADS] = reinterpret_cast<double(*)[NV + 1][SWEEP_THREADS]>(stg_);
+  // Ring of four cells (cell m in slot m & 3) and of two face fields: a
+  // cell's three readers take it from shared memory, so that no cell is live
+  // in registers across the Riemann solver (FP64 256^3, with the straight-line
+  // HLLD: y 1097 -> 925, z 1170 -> 929 us).  Parking the edge value and the
+  // flux there too measured slower (1044: less L1 for what spills).
+  double(*sv)[NV][SWEEP_THREADS] = reinterpret_cast<double(*)[NV][SWEEP_THREADS]>(stg_);
+  double(*sb)[SWEEP_THREADS] =
+      reinterpret_cast<double(*)[SWEEP_THREADS]>(stg_ + 4 * NV * SWEEP_THREADS);
   const int nd = (DIR == 1) ? g.ny : g.nz;
   const long long n = g.n;
   const R gamma = (R)a.gamma;
@@ -1009,73 +1051,76 @@ __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3
                                       : i + (long long)g.nx * t;
     const int m0 = seg * S;
     const int m1 = min(m0 + S, nd);
-    auto stage = [&](int mcell, int mface, int b) {
-      const long long cc = base + (long long)gidx(mcell, nd, g.outflow, DIR) * stride;
+    auto stage_cell = [&](int m) {
+      const long long cc = base + (long long)gidx(m, nd, g.outflow, DIR) * stride;
 #pragma unroll
-      for (int nv = 0; nv < NV; nv++) cp_async8(&stg[b][nv][tid], a.V + nv * n + cc);
-      if constexpr (PHYS != PHYS_HD)
-        cp_async8(&stg[b][NV][tid], a.Bs[DIR] + base + (long long)gidx(mface, nd, g.outflow, DIR) * stride);
-      cp_async_commit();
+      for (int nv = 0; nv < NV; nv++) cp_async8(&sv[m & 3][nv][tid], a.V + nv * n + cc);
     };
-    stage(m0 + 1, m0, 0);
-    R Vp[NV], Vc[NV], vLn[NV], Fp[NV], cmp = R(0);
+    auto stage_face = [&](int m) {
+      if constexpr (PHYS != PHYS_HD)
+        cp_async8(&sb[m & 1][tid],
+                  a.Bs[DIR] + base + (long long)gidx(m, nd, g.outflow, DIR) * stride);
+    };
+    auto cell = [&](int m, R* v) {
+#pragma unroll
+      for (int nv = 0; nv < NV; nv++) v[nv] = (R)sv[m & 3][nv][tid];
+    };
+    stage_cell(m0 - 1);
+    stage_cell(m0);
+    cp_async_commit();
+    stage_cell(m0 + 1);
+    stage_face(m0);
+    cp_async_commit();
+    // FP32 cells (half the registers) are converted once and stay in a window
+    constexpr bool kWindow = sizeof(R) == 4;
+    R vLn[NV], Fp[NV], cmp = R(0), W0[NV], W1[NV];
     {
-      R vmm[NV];
-      load_cell<NV>(a.V, n, base + gidx(m0 - 2, nd, g.outflow, DIR) * stride, vmm);
-      load_cell<NV>(a.V, n, base + gidx(m0 - 1, nd, g.outflow, DIR) * stride, Vp);
-      load_cell<NV>(a.V, n, base + (long long)m0 * stride, Vc);
-      R vrp[NV];
-      if constexpr (three_point<LIM>()) {
-        const R dx = (R)a.dx[DIR];
-#pragma unroll
-        for (int nv = 0; nv < NV; nv++) {
-          vLn[nv] = edge3<LIM>(vmm[nv], Vp[nv], Vc[nv], dx);
-          vrp[nv] = edge3<LIM>(Vc[nv], Vp[nv], vmm[nv], dx);
-          Fp[nv] = R(0);
-        }
-        const R qm[2] = {vmm[RHO], vmm[NV - 1]}, qp[2] = {Vc[RHO], Vc[NV - 1]};
-        mp5_fallback<PHYS, NV>(Vp, qm, qp, vrp, vLn);
-      } else {
-#pragma unroll
-        for (int nv = 0; nv < NV; nv++) {
-          R dv = limit<LIM>(Vc[nv] - Vp[nv], Vp[nv] - vmm[nv]);
-          vLn[nv] = Vp[nv] + R(0.5) * dv;
-          vrp[nv] = Vp[nv] - R(0.5) * dv;
-          Fp[nv] = R(0);
-        }
-        if constexpr (PHYS == PHYS_RMHD) rmhd_vel_limit<NV>(Vp, vrp, vLn);
-      }
-    }
-    int buf = 0;
-    for (int m = m0; m <= m1; m++, buf ^= 1) {
-      stage(m + 2, m + 1, buf ^ 1);   // prefetch for the next iteration
+      R vm[NV], v0[NV], vp[NV], w[NV];
+      load_cell<NV>(a.V, n, base + gidx(m0 - 2, nd, g.outflow, DIR) * stride, vm);
       cp_async_wait1();
-      R Vn[NV], vL[NV], vR[NV], F[NV];
-      if constexpr (three_point<LIM>()) {
-        const R dx = (R)a.dx[DIR];
+      cell(m0 - 1, v0);
+      cell(m0, vp);
+      if constexpr (kWindow) {
 #pragma unroll
         for (int nv = 0; nv < NV; nv++) {
-          Vn[nv] = (R)stg[buf][nv][tid];
-          vL[nv] = vLn[nv];
-          vR[nv] = edge3<LIM>(Vn[nv], Vc[nv], Vp[nv], dx);
-          vLn[nv] = edge3<LIM>(Vp[nv], Vc[nv], Vn[nv], dx);
+          W0[nv] = v0[nv];
+          W1[nv] = vp[nv];
         }
-        const R qm[2] = {Vp[RHO], Vp[NV - 1]}, qp[2] = {Vn[RHO], Vn[NV - 1]};
-        mp5_fallback<PHYS, NV>(Vc, qm, qp, vR, vLn);
-      } else {
+      }
+      cell_edges<PHYS, NV, LIM>(vm, v0, vp, (R)a.dx[DIR], w, vLn);
 #pragma unroll
-        for (int nv = 0; nv < NV; nv++) {
-          Vn[nv] = (R)stg[buf][nv][tid];
-          R dv = limit<LIM>(Vn[nv] - Vc[nv], Vc[nv] - Vp[nv]);
-          vL[nv] = vLn[nv];
-          vR[nv] = Vc[nv] - R(0.5) * dv;
-          vLn[nv] = Vc[nv] + R(0.5) * dv;
+      for (int nv = 0; nv < NV; nv++) Fp[nv] = R(0);
+    }
+    for (int m = m0; m <= m1; m++) {
+      if (m < m1) {   // prefetch for the next iteration
+        stage_cell(m + 2);
+        stage_face(m + 1);
+      }
+      cp_async_commit();
+      cp_async_wait1();
+      R vL[NV], vR[NV], F[NV];
+      {
+        R vm[NV], v0[NV], vp[NV];
+        cell(m + 1, vp);
+        if constexpr (kWindow) {
+#pragma unroll
+          for (int nv = 0; nv < NV; nv++) {
+            vm[nv] = W0[nv];
+            v0[nv] = W1[nv];
+            W0[nv] = v0[nv];
+            W1[nv] = vp[nv];
+          }
+        } else {
+          cell(m - 1, vm);
+          cell(m, v0);
         }
-        if constexpr (PHYS == PHYS_RMHD) rmhd_vel_limit<NV>(Vc, vR, vLn);
+#pragma unroll
+        for (int nv = 0; nv < NV; nv++) vL[nv] = vLn[nv];
+        cell_edges<PHYS, NV, LIM>(vm, v0, vp, (R)a.dx[DIR], vR, vLn);
       }
       R Bn = R(0);
       if constexpr (PHYS != PHYS_HD) {
-        Bn = (R)stg[buf][NV][tid];
+        Bn = (R)sb[m & 1][tid];
         vL[BX1 + DIR] = Bn;
         vR[BX1 + DIR] = Bn;
       }
@@ -1093,11 +1138,7 @@ __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3
         cell_update<PHYS, NV, NDIM>(a, n, base + (long long)(m - 1) * stride, Fp, F, cmp, cm,
                                     DIR);
 #pragma unroll
-      for (int nv = 0; nv < NV; nv++) {
-        Vp[nv] = Vc[nv];
-        Vc[nv] = Vn[nv];
-        Fp[nv] = F[nv];
-      }
+      for (int nv = 0; nv < NV; nv++) Fp[nv] = F[nv];
       cmp = cm;
     }
     cp_async_wait0();
@@ -1105,26 +1146,26 @@ __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3
   if (err) atomicOr(a.err, err);
 }
 
-// t is the transverse index (k for DIR=1, j for DIR=2).  FLAT = false:
-// grid (x-blocks, t * nseg + seg), the block's columns share one t.  FLAT =
-// true (nx not a multiple of the block): a 1-D grid of (column block cb,
-// segment) pairs, segments innermost, with the (x, t) columns numbered
-// together (col = cb * SWEEP_THREADS + thread, i = col % nx, t = col / nx),
-// so that no block is part-empty.
-template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, typename R,
-          typename CTT, bool FLAT>
+// t is the transverse index (k for DIR=1, j for DIR=2).  Grid (x-blocks,
+// t * nseg + seg), the block's columns sharing one t; with `flat` (nx not a
+// multiple of the block) a 1-D grid of (column block cb, segment) pairs,
+// segments innermost, with the (x, t) columns numbered together (col = cb *
+// SWEEP_THREADS + thread, i = col % nx, t = col / nx), so that no block is
+// part-empty.
+template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, typename R, typename CTT>
 __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_m_minb<PHYS, R>()))
-    sweep_m_kernel(StageArgs<CTT> a, Grid3 g, int S) {
-  __shared__ double stg[sweep_m_stage_doubles<NV>()];
+    sweep_m_kernel(StageArgs<CTT> a, Grid3 g, int S, bool flat) {
+  __shared__ double stg[sweep_m_stage_doubles<NV, LIM>()];
   const int nd = (DIR == 1) ? g.ny : g.nz;
   const int nseg = (nd + S - 1) / S;
   int i, t, seg;
-  if constexpr (FLAT) {
+  if (flat) {
     const int nt = (DIR == 1) ? g.nz : g.ny;
     seg = (int)(blockIdx.x % (unsigned)nseg);
-    const int col = (int)(blockIdx.x / (unsigned)nseg) * SWEEP_THREADS + (int)threadIdx.x;
-    i = col % g.nx;
-    t = col / g.nx;
+    const long long col =
+        (long long)(blockIdx.x / (unsigned)nseg) * SWEEP_THREADS + (int)threadIdx.x;
+    t = (int)(col / g.nx);
+    i = (int)(col - (long long)t * g.nx);
     if (t >= nt) i = g.nx;   // past the last column: the thread stays idle
   } else {
     i = blockIdx.x * SWEEP_THREADS + threadIdx.x;
@@ -1177,14 +1218,23 @@ __device__ __forceinline__ void uct_terms(const R* b, const R* q, R aL, R aR, R 
     vL = q[1] + p1;
     vR = q[2] + m2;
   } else {
-    R dbl = limit<LIM_MC>(b[2] - b[1], b[1] - b[0]);
-    R dbr = limit<LIM_MC>(b[3] - b[2], b[2] - b[1]);
-    R dql = limit<LIM>(q[2] - q[1], q[1] - q[0]);
-    R dqr = limit<LIM>(q[3] - q[2], q[2] - q[1]);
-    bL = b[1] + R(0.5) * dbl;
-    bR = b[2] - R(0.5) * dbr;
-    vL = q[1] + R(0.5) * dql;
-    vR = q[2] - R(0.5) * dqr;
+    if constexpr (sizeof(R) == 8) {
+      // half_limit saves two products a slope (tile kernel 841 -> 705 us at
+      // 256^3); in the FP32 march kernel it measured slower (517 -> 593)
+      bL = b[1] + half_limit<LIM_MC>(b[2] - b[1], b[1] - b[0]);
+      bR = b[2] - half_limit<LIM_MC>(b[3] - b[2], b[2] - b[1]);
+      vL = q[1] + half_limit<LIM>(q[2] - q[1], q[1] - q[0]);
+      vR = q[2] - half_limit<LIM>(q[3] - q[2], q[2] - q[1]);
+    } else {
+      R dbl = limit<LIM_MC>(b[2] - b[1], b[1] - b[0]);
+      R dbr = limit<LIM_MC>(b[3] - b[2], b[2] - b[1]);
+      R dql = limit<LIM>(q[2] - q[1], q[1] - q[0]);
+      R dqr = limit<LIM>(q[3] - q[2], q[2] - q[1]);
+      bL = b[1] + R(0.5) * dbl;
+      bR = b[2] - R(0.5) * dbr;
+      vL = q[1] + R(0.5) * dql;
+      vR = q[2] - R(0.5) * dqr;
+    }
   }
   phi = dR * bR - dL * bL;
   avg = aL * vL * bL + aR * vR * bR;

@@ -13,12 +13,13 @@
 #ifndef GP_MIXED
 #define GP_MIXED 0
 #endif
-// GP_PART selects the schemes this unit instantiates (0 HD, 1 MHD with
-// HLLD/HLL, 2 RMHD, 3 MHD with Lax-Friedrichs/HLLC), so that the build
-// compiles the four in parallel; the entry points
+// GP_PART selects the schemes this unit instantiates (0 HD, 1 MHD HLLD with
+// the upwind EMFs, 2 RMHD HLLD, 3 MHD with Lax-Friedrichs/HLLC, 4 RMHD with
+// HLL/Lax-Friedrichs, 5 the other MHD HLLD and HLL schemes), so that the build
+// compiles them in parallel; the entry points
 // launch_stage_{fp64,mixed}_p<part> are joined by gp_launch_dispatch.cu.
 #ifndef GP_PART
-#error "compile gp_launch.cu with -DGP_PART=0, 1, 2 or 3"
+#error "compile gp_launch.cu with -DGP_PART=0 .. 5"
 #endif
 #define GP_CAT2(a, b) a##b
 #define GP_CAT(a, b) GP_CAT2(a, b)
@@ -55,7 +56,7 @@ static StageArgs<CTT> make_args(const StageDesc& d) {
   a.Uout = d.Uout;
   a.Vout = d.Vout;
   a.gamma = d.gamma;
-  a.inv_gm1 = fixed_inv(d.gamma - 1.0);
+  a.inv_gm1 = gamma_inv(d.gamma);
   a.small_rho = d.small_rho;
   a.small_prs = d.small_prs;
   a.stage = d.stage;
@@ -67,8 +68,70 @@ static StageArgs<CTT> make_args(const StageDesc& d) {
   return a;
 }
 
+// Parts an x-row is swept in.  A warp solves 32 faces at a time and a part
+// one face more than its cells, so k chunks hold 32 k - 1 cells; a whole
+// periodic row needs no extra face.  The count with the fewest (waves of
+// resident warps) x (chunks, + 1 for the start-up) is taken: one for grids
+// that fill the SMs with whole rows.
+template <int PHYS, int LIM, typename R>
+static int x_segments(int nx, long long rows) {
+  if (LIM == LIM_PPM || five_point<LIM>()) return 1;
+  const long long resident = 148LL * sweep_x_minb<PHYS, R>() * (SWEEP_THREADS / 32);
+  auto cost = [&](int nseg, int chunks) {
+    return (rows * nseg + resident - 1) / resident * (chunks + 1);
+  };
+  int best = 1;
+  long long c = cost(1, (nx + 31) / 32);
+  for (int k = (nx + 31) / 32; k >= 1; k--) {
+    const int nseg = (nx + 32 * k - 2) / (32 * k - 1);
+    if (nseg > 1 && cost(nseg, k) < c) {
+      c = cost(nseg, k);
+      best = nseg;
+    }
+  }
+  return best;
+}
+
+// Cells a thread of a y or z sweep marches over, for `cols` blocks of columns
+// of nd cells: the length with the fewest (waves of resident blocks) x (cells
+// marched, + 2 for the start-up and the face at the end).  A last wave that
+// fills few SMs costs a whole wave, and a grid that does not fill them takes
+// the shortest march.
+template <int PHYS, typename R>
+static int march_length(long long cols, int nd) {
+  const long long resident = 148LL * sweep_m_minb<PHYS, R>();
+  int best = 1;
+  long long c = 0;
+  for (int len = 1; len <= nd && len <= 128; len++) {
+    const int nseg = (nd + len - 1) / len;
+    const long long q = (cols * nseg + resident - 1) / resident * (len + 2);
+    if (len == 1 || q <= c) {
+      c = q;
+      best = len;
+    }
+  }
+  return best;
+}
+
+// y or z sweep over nt transverse positions of nd cells: grid (x-blocks,
+// transverse index x pencil segments); when nx is not a multiple of the
+// block, a 1-D grid over (x, transverse) columns numbered together, so that
+// no block is part-empty.
+template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, typename F1, typename F2>
+static void launch_m(const StageArgs<CTT>& a, const Grid3& g, int nt, int nd, cudaStream_t s,
+                     F1& pre, F2& post) {
+  const long long cols = ((long long)g.nx * nt + SWEEP_THREADS - 1) / SWEEP_THREADS;
+  const int seg = march_length<PHYS, RT>(cols, nd);
+  const int nseg = (nd + seg - 1) / seg;
+  pre();
+  const bool flat = g.nx % SWEEP_THREADS != 0 || (long long)nt * nseg > 65535;
+  const dim3 grid = flat ? dim3((unsigned)(cols * nseg)) : dim3(g.nx / SWEEP_THREADS, nt * nseg);
+  sweep_m_kernel<PHYS, NV, NDIM, RS, CT, LIM, DIR, RT, CTT><<<grid, SWEEP_THREADS, 0, s>>>(a, g, seg, flat);
+  post();
+}
+
 template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM>
-static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, int seg, cudaStream_t s,
+static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, cudaStream_t s,
                       cudaEvent_t* ev) {
   Grid3 g{gd.nx, gd.ny, gd.nz, gd.n, gd.outflow};
   for (int d = 0; d < 3; d++) {
@@ -83,38 +146,15 @@ static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, int seg, cuda
   {
     const int rows = gd.ny * gd.nz;
     const int wpb = SWEEP_THREADS / 32;
-    dim3 grid((rows + wpb - 1) / wpb);
+    const int nseg = x_segments<PHYS, LIM, RT>(gd.nx, rows);
+    dim3 grid((unsigned)(((long long)rows * nseg + wpb - 1) / wpb));
     pre();
-    sweep_x_kernel<PHYS, NV, NDIM, RS, CT, LIM, RT, CTT><<<grid, SWEEP_THREADS, 0, s>>>(a, g);
+    sweep_x_kernel<PHYS, NV, NDIM, RS, CT, LIM, RT, CTT><<<grid, SWEEP_THREADS, 0, s>>>(a, g, nseg);
     post();
   }
-  // y/z sweeps: grid (x-blocks, transverse index x pencil segments); when
-  // nx is not a multiple of the block, a 1-D grid over (x, transverse)
-  // columns numbered together, so that no block is part-empty (FLAT)
-  const bool flat = gd.nx % SWEEP_THREADS != 0;
-  auto grid_m = [&](int nt, int nseg) {
-    if (flat)
-      return dim3((unsigned)(((long long)gd.nx * nt + SWEEP_THREADS - 1) / SWEEP_THREADS * nseg));
-    return dim3(gd.nx / SWEEP_THREADS, nt * nseg);
-  };
-  {
-    const dim3 grid = grid_m(gd.nz, (gd.ny + seg - 1) / seg);
-    pre();
-    if (flat)
-      sweep_m_kernel<PHYS, NV, NDIM, RS, CT, LIM, 1, RT, CTT, true><<<grid, SWEEP_THREADS, 0, s>>>(a, g, seg);
-    else
-      sweep_m_kernel<PHYS, NV, NDIM, RS, CT, LIM, 1, RT, CTT, false><<<grid, SWEEP_THREADS, 0, s>>>(a, g, seg);
-    post();
-  }
-  if constexpr (NDIM == 3) {
-    const dim3 grid = grid_m(gd.ny, (gd.nz + seg - 1) / seg);
-    pre();
-    if (flat)
-      sweep_m_kernel<PHYS, NV, NDIM, RS, CT, LIM, 2, RT, CTT, true><<<grid, SWEEP_THREADS, 0, s>>>(a, g, seg);
-    else
-      sweep_m_kernel<PHYS, NV, NDIM, RS, CT, LIM, 2, RT, CTT, false><<<grid, SWEEP_THREADS, 0, s>>>(a, g, seg);
-    post();
-  }
+  launch_m<PHYS, NV, NDIM, RS, CT, LIM, 1>(a, g, gd.nz, gd.ny, s, pre, post);
+  if constexpr (NDIM == 3) 
+    launch_m<PHYS, NV, NDIM, RS, CT, LIM, 2>(a, g, gd.ny, gd.nz, s, pre, post);
   const unsigned nb = (unsigned)((gd.n + 255) / 256);
   if constexpr (PHYS != PHYS_HD) {
     pre();
@@ -154,108 +194,107 @@ static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, int seg, cuda
 }
 
 template <int PHYS, int NV, int NDIM, int RS, int CT>
-static int by_lim(const StageArgs<CTT>& a, const GridDims& g, int lim, int seg, cudaStream_t s,
+static int by_lim(const StageArgs<CTT>& a, const GridDims& g, int lim, cudaStream_t s,
                   cudaEvent_t* ev) {
   switch (lim) {
-    case LIM_MC: run_stage<PHYS, NV, NDIM, RS, CT, LIM_MC>(a, g, seg, s, ev); return 0;
-    case LIM_VL: run_stage<PHYS, NV, NDIM, RS, CT, LIM_VL>(a, g, seg, s, ev); return 0;
-    case LIM_MINMOD: run_stage<PHYS, NV, NDIM, RS, CT, LIM_MINMOD>(a, g, seg, s, ev); return 0;
-    case LIM_PPM: run_stage<PHYS, NV, NDIM, RS, CT, LIM_PPM>(a, g, seg, s, ev); return 0;
-    case LIM_MP5: run_stage<PHYS, NV, NDIM, RS, CT, LIM_MP5>(a, g, seg, s, ev); return 0;
-    case LIM_WENOZ: run_stage<PHYS, NV, NDIM, RS, CT, LIM_WENOZ>(a, g, seg, s, ev); return 0;
-    case LIM_LIMO3: run_stage<PHYS, NV, NDIM, RS, CT, LIM_LIMO3>(a, g, seg, s, ev); return 0;
-    case LIM_WENO3: run_stage<PHYS, NV, NDIM, RS, CT, LIM_WENO3>(a, g, seg, s, ev); return 0;
-    case LIM_FLAT: run_stage<PHYS, NV, NDIM, RS, CT, LIM_FLAT>(a, g, seg, s, ev); return 0;
+    case LIM_MC: run_stage<PHYS, NV, NDIM, RS, CT, LIM_MC>(a, g, s, ev); return 0;
+    case LIM_VL: run_stage<PHYS, NV, NDIM, RS, CT, LIM_VL>(a, g, s, ev); return 0;
+    case LIM_MINMOD: run_stage<PHYS, NV, NDIM, RS, CT, LIM_MINMOD>(a, g, s, ev); return 0;
+    case LIM_PPM: run_stage<PHYS, NV, NDIM, RS, CT, LIM_PPM>(a, g, s, ev); return 0;
+    case LIM_MP5: run_stage<PHYS, NV, NDIM, RS, CT, LIM_MP5>(a, g, s, ev); return 0;
+    case LIM_WENOZ: run_stage<PHYS, NV, NDIM, RS, CT, LIM_WENOZ>(a, g, s, ev); return 0;
+    case LIM_LIMO3: run_stage<PHYS, NV, NDIM, RS, CT, LIM_LIMO3>(a, g, s, ev); return 0;
+    case LIM_WENO3: run_stage<PHYS, NV, NDIM, RS, CT, LIM_WENO3>(a, g, s, ev); return 0;
+    case LIM_FLAT: run_stage<PHYS, NV, NDIM, RS, CT, LIM_FLAT>(a, g, s, ev); return 0;
     case LIM_VANALBADA:
-      run_stage<PHYS, NV, NDIM, RS, CT, LIM_VANALBADA>(a, g, seg, s, ev);
+      run_stage<PHYS, NV, NDIM, RS, CT, LIM_VANALBADA>(a, g, s, ev);
       return 0;
-    case LIM_OSPRE: run_stage<PHYS, NV, NDIM, RS, CT, LIM_OSPRE>(a, g, seg, s, ev); return 0;
-    case LIM_UMIST: run_stage<PHYS, NV, NDIM, RS, CT, LIM_UMIST>(a, g, seg, s, ev); return 0;
+    case LIM_OSPRE: run_stage<PHYS, NV, NDIM, RS, CT, LIM_OSPRE>(a, g, s, ev); return 0;
+    case LIM_UMIST: run_stage<PHYS, NV, NDIM, RS, CT, LIM_UMIST>(a, g, s, ev); return 0;
     default: return -1;
   }
 }
 
 template <int NDIM>
-static int by_scheme(const StageArgs<CTT>& a, const GridDims& g, const SchemeKey& k, int seg,
+static int by_scheme(const StageArgs<CTT>& a, const GridDims& g, const SchemeKey& k,
                      cudaStream_t s, cudaEvent_t* ev) {
 #if GP_PART == 1
-  // MHD with the HLLD and HLL solvers
-  if (k.physics == PHYS_MHD && k.ct == CT_CONTACT) {
-    if (k.riemann == RS_HLLD)
-      return by_lim<PHYS_MHD, 8, NDIM, RS_HLLD, CT_CONTACT>(a, g, k.limiter, seg, s, ev);
-    if (k.riemann == RS_HLL)
-      return by_lim<PHYS_MHD, 8, NDIM, RS_HLL, CT_CONTACT>(a, g, k.limiter, seg, s, ev);
-    return -1;
+  if (k.physics == PHYS_MHD && k.riemann == RS_HLLD) {
+    if (k.ct == CT_UCT_HLLD)
+      return by_lim<PHYS_MHD, 8, NDIM, RS_HLLD, CT_UCT_HLLD>(a, g, k.limiter, s, ev);
+    if (k.ct == CT_UCT_HLL)
+      return by_lim<PHYS_MHD, 8, NDIM, RS_HLLD, CT_UCT_HLL>(a, g, k.limiter, s, ev);
   }
-  if (k.physics == PHYS_MHD && k.ct == CT_ARITH) {
-    if (k.riemann == RS_HLLD)
-      return by_lim<PHYS_MHD, 8, NDIM, RS_HLLD, CT_ARITH>(a, g, k.limiter, seg, s, ev);
-    if (k.riemann == RS_HLL)
-      return by_lim<PHYS_MHD, 8, NDIM, RS_HLL, CT_ARITH>(a, g, k.limiter, seg, s, ev);
-    return -1;
+#endif
+#if GP_PART == 5
+  if (k.physics == PHYS_MHD && k.riemann == RS_HLLD) {
+    if (k.ct == CT_CONTACT)
+      return by_lim<PHYS_MHD, 8, NDIM, RS_HLLD, CT_CONTACT>(a, g, k.limiter, s, ev);
+    if (k.ct == CT_ARITH)
+      return by_lim<PHYS_MHD, 8, NDIM, RS_HLLD, CT_ARITH>(a, g, k.limiter, s, ev);
   }
-  if (k.physics == PHYS_MHD) {
-    if (k.riemann == RS_HLLD && k.ct == CT_UCT_HLLD)
-      return by_lim<PHYS_MHD, 8, NDIM, RS_HLLD, CT_UCT_HLLD>(a, g, k.limiter, seg, s, ev);
-    if (k.riemann == RS_HLLD && k.ct == CT_UCT_HLL)
-      return by_lim<PHYS_MHD, 8, NDIM, RS_HLLD, CT_UCT_HLL>(a, g, k.limiter, seg, s, ev);
-    if (k.riemann == RS_HLL && k.ct == CT_UCT_HLL)
-      return by_lim<PHYS_MHD, 8, NDIM, RS_HLL, CT_UCT_HLL>(a, g, k.limiter, seg, s, ev);
-    return -1;
+  if (k.physics == PHYS_MHD && k.riemann == RS_HLL) {
+    if (k.ct == CT_CONTACT)
+      return by_lim<PHYS_MHD, 8, NDIM, RS_HLL, CT_CONTACT>(a, g, k.limiter, s, ev);
+    if (k.ct == CT_ARITH)
+      return by_lim<PHYS_MHD, 8, NDIM, RS_HLL, CT_ARITH>(a, g, k.limiter, s, ev);
+    if (k.ct == CT_UCT_HLL)
+      return by_lim<PHYS_MHD, 8, NDIM, RS_HLL, CT_UCT_HLL>(a, g, k.limiter, s, ev);
   }
 #endif
 #if GP_PART == 3
   // MHD with the Lax-Friedrichs and HLLC solvers (UCT_HLL, ARITHMETIC or CT_CONTACT)
   if (k.physics == PHYS_MHD && k.ct == CT_CONTACT) {
     if (k.riemann == RS_TVDLF)
-      return by_lim<PHYS_MHD, 8, NDIM, RS_TVDLF, CT_CONTACT>(a, g, k.limiter, seg, s, ev);
+      return by_lim<PHYS_MHD, 8, NDIM, RS_TVDLF, CT_CONTACT>(a, g, k.limiter, s, ev);
     if (k.riemann == RS_HLLC)
-      return by_lim<PHYS_MHD, 8, NDIM, RS_HLLC, CT_CONTACT>(a, g, k.limiter, seg, s, ev);
+      return by_lim<PHYS_MHD, 8, NDIM, RS_HLLC, CT_CONTACT>(a, g, k.limiter, s, ev);
     return -1;
   }
   if (k.physics == PHYS_MHD && k.ct == CT_ARITH) {
     if (k.riemann == RS_TVDLF)
-      return by_lim<PHYS_MHD, 8, NDIM, RS_TVDLF, CT_ARITH>(a, g, k.limiter, seg, s, ev);
+      return by_lim<PHYS_MHD, 8, NDIM, RS_TVDLF, CT_ARITH>(a, g, k.limiter, s, ev);
     if (k.riemann == RS_HLLC)
-      return by_lim<PHYS_MHD, 8, NDIM, RS_HLLC, CT_ARITH>(a, g, k.limiter, seg, s, ev);
+      return by_lim<PHYS_MHD, 8, NDIM, RS_HLLC, CT_ARITH>(a, g, k.limiter, s, ev);
     return -1;
   }
   if (k.physics == PHYS_MHD) {
     if (k.riemann == RS_TVDLF && k.ct == CT_UCT_HLL)
-      return by_lim<PHYS_MHD, 8, NDIM, RS_TVDLF, CT_UCT_HLL>(a, g, k.limiter, seg, s, ev);
+      return by_lim<PHYS_MHD, 8, NDIM, RS_TVDLF, CT_UCT_HLL>(a, g, k.limiter, s, ev);
     if (k.riemann == RS_HLLC && k.ct == CT_UCT_HLL)
-      return by_lim<PHYS_MHD, 8, NDIM, RS_HLLC, CT_UCT_HLL>(a, g, k.limiter, seg, s, ev);
+      return by_lim<PHYS_MHD, 8, NDIM, RS_HLLC, CT_UCT_HLL>(a, g, k.limiter, s, ev);
     return -1;
   }
 #endif
 #if GP_PART == 2
-  if (k.physics == PHYS_RMHD) {
-    if (k.riemann == RS_HLLD && k.ct == CT_UCT_HLL)
-      return by_lim<PHYS_RMHD, 8, NDIM, RS_HLLD, CT_UCT_HLL>(a, g, k.limiter, seg, s, ev);
-    if (k.riemann == RS_HLL && k.ct == CT_UCT_HLL)
-      return by_lim<PHYS_RMHD, 8, NDIM, RS_HLL, CT_UCT_HLL>(a, g, k.limiter, seg, s, ev);
-    if (k.riemann == RS_TVDLF && k.ct == CT_UCT_HLL)
-      return by_lim<PHYS_RMHD, 8, NDIM, RS_TVDLF, CT_UCT_HLL>(a, g, k.limiter, seg, s, ev);
-    return -1;
+  if (k.physics == PHYS_RMHD && k.riemann == RS_HLLD && k.ct == CT_UCT_HLL)
+    return by_lim<PHYS_RMHD, 8, NDIM, RS_HLLD, CT_UCT_HLL>(a, g, k.limiter, s, ev);
+#endif
+#if GP_PART == 4
+  if (k.physics == PHYS_RMHD && k.ct == CT_UCT_HLL) {
+    if (k.riemann == RS_HLL)
+      return by_lim<PHYS_RMHD, 8, NDIM, RS_HLL, CT_UCT_HLL>(a, g, k.limiter, s, ev);
+    if (k.riemann == RS_TVDLF)
+      return by_lim<PHYS_RMHD, 8, NDIM, RS_TVDLF, CT_UCT_HLL>(a, g, k.limiter, s, ev);
   }
 #endif
 #if GP_PART == 0
   if (k.physics == PHYS_HD) {
-    if (k.riemann == RS_HLLC) return by_lim<PHYS_HD, 5, NDIM, RS_HLLC, 0>(a, g, k.limiter, seg, s, ev);
-    if (k.riemann == RS_HLL) return by_lim<PHYS_HD, 5, NDIM, RS_HLL, 0>(a, g, k.limiter, seg, s, ev);
+    if (k.riemann == RS_HLLC) return by_lim<PHYS_HD, 5, NDIM, RS_HLLC, 0>(a, g, k.limiter, s, ev);
+    if (k.riemann == RS_HLL) return by_lim<PHYS_HD, 5, NDIM, RS_HLL, 0>(a, g, k.limiter, s, ev);
     if (k.riemann == RS_TVDLF)
-      return by_lim<PHYS_HD, 5, NDIM, RS_TVDLF, 0>(a, g, k.limiter, seg, s, ev);
+      return by_lim<PHYS_HD, 5, NDIM, RS_TVDLF, 0>(a, g, k.limiter, s, ev);
     return -1;
   }
 #endif
   return -1;
 }
 
-int GP_LAUNCH_STAGE(const StageDesc& d, const GridDims& g, const SchemeKey& k, int seg,
+int GP_LAUNCH_STAGE(const StageDesc& d, const GridDims& g, const SchemeKey& k,
                     cudaStream_t s, cudaEvent_t* ev) {
   StageArgs<CTT> a = make_args(d);
-  if (k.ndim == 2) return by_scheme<2>(a, g, k, seg, s, ev);
-  if (k.ndim == 3) return by_scheme<3>(a, g, k, seg, s, ev);
+  if (k.ndim == 2) return by_scheme<2>(a, g, k, s, ev);
+  if (k.ndim == 3) return by_scheme<3>(a, g, k, s, ev);
   return -1;
 }
 

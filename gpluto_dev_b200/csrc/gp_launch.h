@@ -47,17 +47,13 @@ struct SchemeKey {
 // `ev` (may be null) receives an event pair around every kernel launch, in
 // launch order (2*stage_launch_count(k) events).
 int launch_stage_fp64(const StageDesc& d, const GridDims& g, const SchemeKey& k,
-                      int seg, cudaStream_t s, cudaEvent_t* ev);
+                      cudaStream_t s, cudaEvent_t* ev);
 int launch_stage_mixed(const StageDesc& d, const GridDims& g, const SchemeKey& k,
-                       int seg, cudaStream_t s, cudaEvent_t* ev);
+                       cudaStream_t s, cudaEvent_t* ev);
 int launch_prim2cons(int physics, const double* V, double* U, long long n, double gamma,
                      cudaStream_t s);
 // Sets the text returned by gp_last_error on this thread; returns `code`.
 int set_last_error(int code, const char* msg);
-
-// Resident blocks per SM the y/z marching sweeps are compiled for
-// (SWEEP_THREADS threads each).
-int sweep_m_blocks_per_sm(int physics, bool mixed);
 
 // Number of kernel launches one stage issues for this scheme, and their names.
 int stage_launch_count(const SchemeKey& k);

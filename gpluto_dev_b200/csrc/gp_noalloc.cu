@@ -156,14 +156,9 @@ extern "C" int gp_advance_step_noalloc(const gp_grid_desc* grid, const gp_scheme
   const bool ppm = scheme->reconstruction == GP_REC_PARABOLIC;
   gp::SchemeKey key{scheme->physics, ndim, scheme->riemann, scheme->ct_emf,
                     ppm ? 4 /* LIM_PPM */ : scheme->limiter};
-  int seg = 64;
-  {
-    const long long cols = (long long)nx * (ndim == 3 ? nz : 1);
-    while (seg > 4 && cols * ((ny + seg - 1) / seg) < 148LL * 1024) seg /= 2;
-  }
   auto launch = [&](const gp::StageDesc& sd) {
-    return mixed ? gp::launch_stage_mixed(sd, g, key, seg, s, nullptr)
-                 : gp::launch_stage_fp64(sd, g, key, seg, s, nullptr);
+    return mixed ? gp::launch_stage_mixed(sd, g, key, s, nullptr)
+                 : gp::launch_stage_fp64(sd, g, key, s, nullptr);
   };
   // stage 1: (U, B) -> (U1, B1)
   d.stage = 1;

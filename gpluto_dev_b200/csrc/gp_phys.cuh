@@ -10,6 +10,7 @@
 // Riemann fluxes; the callers keep accumulation in FP64).
 #pragma once
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 #include "gp_exact.cuh"
@@ -97,6 +98,23 @@ __device__ __forceinline__ R limit(R dvp, R dvm) {
     return R(0);
   } else {
     return R(0);
+  }
+}
+
+// Half the limited slope, as the edge values take it (v -+ 0.5 * slope).  MC:
+// 0.5 * (0.5 s) = 0.25 s and 0.5 * (2 m) = m, and halving both sides keeps
+// the comparison; nothing underflows where the product of the differences is
+// positive (their sum is then at least 2^-537, 2^-75 in FP32), so the values
+// are the same.
+template <int LIM, typename R>
+__device__ __forceinline__ R half_limit(R dvp, R dvm) {
+  if constexpr (LIM == LIM_MC) {
+    const R q = R(0.25) * (dvm + dvp);
+    const R m = rabs(dvp) < rabs(dvm) ? dvp : dvm;
+    const R h = rabs(q) < rabs(m) ? q : m;
+    return dvp * dvm > R(0) ? h : R(0);
+  } else {
+    return R(0.5) * limit<LIM>(dvp, dvm);
   }
 }
 
@@ -465,7 +483,7 @@ __device__ __forceinline__ void mhd_prim2cons(const R* v, R* u, R gmm1, R y, A& 
   R kinb2 = v[VX1] * v[VX1] + v[VX1 + 1] * v[VX1 + 1] + v[VX1 + 2] * v[VX1 + 2];
   kinb2 = v[RHO] * kinb2 + v[BX1] * v[BX1] + v[BX2] * v[BX2] + v[BX3] * v[BX3];
   kinb2 *= R(0.5);
-  u[7] = kinb2 + ar.quot_pos(v[7], gmm1, y);
+  u[7] = kinb2 + ar.quot_bpos(v[7], gmm1, y);  // p > 0 in range, as gamma p is
 }
 
 template <int DIR, typename R, typename A>
@@ -479,7 +497,7 @@ __device__ __forceinline__ void mhd_signal_speed(const R* v, R gamma, R& cmin, R
   R Bmag2 = b1 * b1 + Btmag2;
   R cf = gpr - Bmag2;
   cf = gpr + Bmag2 + ar.root(cf * cf + R(4) * gpr * Btmag2);
-  cf = ar.root(ar.quot_pos(R(0.5) * cf, v[RHO], yr));
+  cf = ar.root(ar.quot_bpos(R(0.5) * cf, v[RHO], yr));  // in range if its root is
   cmax = v[VXn] + cf;
   cmin = v[VXn] - cf;
 }
@@ -497,10 +515,6 @@ __device__ __forceinline__ R mhd_hlld_line(const R* vl, const R* vr, R* flux, R 
   constexpr int VXn = VX1 + DIR, VXt = VX1 + (DIR + 1) % 3, VXb = VX1 + (DIR + 2) % 3;
   constexpr int MXn = MX1 + DIR, MXt = MX1 + (DIR + 1) % 3, MXb = MX1 + (DIR + 2) % 3;
   constexpr int BXn = BX1 + DIR, BXt = BX1 + (DIR + 1) % 3, BXb = BX1 + (DIR + 2) % 3;
-  R ul[8], ur[8];
-  const R gmm1 = gamma - R(1);
-  mhd_prim2cons(vl, ul, gmm1, ygm, ar);
-  mhd_prim2cons(vr, ur, gmm1, ygm, ar);
   R Sl, Sr;
   {
     R sl_min, sl_max, sr_min, sr_max;
@@ -515,31 +529,41 @@ __device__ __forceinline__ R mhd_hlld_line(const R* vl, const R* vr, R* flux, R 
   const R Bx = (Sr * vr[BXn] - Sl * vl[BXn]) * dS_1;
   const R sBx = (Bx > R(0) ? R(1) : R(-1));
   const R dul = Sl - vl[VXn], dur = Sr - vr[VXn];
-  const R rdl = ul[RHO] * dul, rdr = ur[RHO] * dur;
-  R scrh = ar.inv_pos(dur * ur[RHO] - dul * ul[RHO]);
-  const R SM = (dur * ur[MXn] - dul * ul[MXn] - ptr + ptl) * scrh;
-  R pts = dur * ur[RHO] * ptl - dul * ul[RHO] * ptr +
+  const R rdl = vl[RHO] * dul, rdr = vr[RHO] * dur;
+  const R mnl = vl[RHO] * vl[VXn], mnr = vr[RHO] * vr[VXn];
+  R scrh = ar.inv_pos(dur * vr[RHO] - dul * vl[RHO]);
+  const R SM = (dur * mnr - dul * mnl - ptr + ptl) * scrh;
+  R pts = dur * vr[RHO] * ptl - dul * vl[RHO] * ptr +
           vl[RHO] * vr[RHO] * dur * dul * (vr[VXn] - vl[VXn]);
   pts *= scrh;
+  // Sl - SM < 0 < Sr - SM (any other sign sets the flag); the star densities
+  // are in range if their roots are
   const R dsl = Sl - SM, dsr = Sr - SM;
-  const R ysl = ar.inv(dsl), ysr = ar.inv_pos(dsr);
-  const R rhosl = ar.quot(rdl, dsl, ysl), rhosr = ar.quot_pos(rdr, dsr, ysr);
+  const R ysl = ar.inv_pos(-dsl), ysr = ar.inv_pos(dsr);
+  const R rhosl = ar.quot_bpos(-rdl, -dsl, ysl), rhosr = ar.quot_bpos(rdr, dsr, ysr);
+  ar.densities(rhosl, rhosr);
   const R sqrL = ar.root(rhosl), sqrR = ar.root(rhosr);
-  const R yqL = ar.inv_pos(sqrL), yqR = ar.inv_pos(sqrR);
-  R S1L = SM - ar.quot(rabs(Bx), sqrL, yqL);
-  R S1R = SM + ar.quot(rabs(Bx), sqrR, yqR);
+  const R yqL = ar.inv_in(sqrL), yqR = ar.inv_in(sqrR);
+  ar.check(Bx);
+  R S1L = SM - ar.quot_bpos(rabs(Bx), sqrL, yqL);
+  R S1R = SM + ar.quot_bpos(rabs(Bx), sqrR, yqR);
 
   if constexpr (CT == CT_UCT_HLLD) {  // ct_store_ucthlld: Sc is SM, the same expression
-    const R Sal = SM - ar.quot(rabs(Bn), sqrL, yqL);
-    const R Sar = SM + ar.quot(rabs(Bn), sqrR, yqR);
-    const R chiL = ar.div((vl[VXn] - SM) * dsl, Sal + Sl - R(2) * SM);
-    const R chiR = ar.div((vr[VXn] - SM) * dsr, Sar + Sr - R(2) * SM);
-    const R nuL = ar.div_pos(Sal + Sl, rabs(Sal) + rabs(Sl));
-    const R nuR = ar.div_pos(Sar + Sr, rabs(Sar) + rabs(Sr));
+    ar.check(Bn);
+    const R Sal = SM - ar.quot_bpos(rabs(Bn), sqrL, yqL);
+    const R Sar = SM + ar.quot_bpos(rabs(Bn), sqrR, yqR);
+    const R chiL = ar.div_any((vl[VXn] - SM) * dsl, Sal + Sl - R(2) * SM);
+    const R chiR = ar.div_any((vr[VXn] - SM) * dsr, Sar + Sr - R(2) * SM);
+    // (x + y) / (|x| + |y|): with the divisor in range the dividend is 0 or
+    // above 2^-255 (terms that cancel are both near half the divisor)
+    const R dnl = rabs(Sal) + rabs(Sl), dnr = rabs(Sar) + rabs(Sr);
+    const R nuL = ar.quot_bpos(Sal + Sl, dnl, ar.inv_pos(dnl));
+    const R nuR = ar.quot_bpos(Sar + Sr, dnr, ar.inv_pos(dnr));
     const bool far = rabs(Sar - Sal) > R(1.e-9) * rabs(Sr - Sl);
     // 0/0 when both vanish, which is not `far`: any divisor will do there
-    const R den = rabs(Sal) + rabs(Sar);
-    const R nuLR = ar.div_pos(Sal + Sar, den > R(0) ? den : R(1));
+    R den = rabs(Sal) + rabs(Sar);
+    den = den > R(0) ? den : R(1);
+    const R nuLR = ar.quot_bpos(Sal + Sar, den, ar.inv_pos(den));
     const R dL = R(0.5) * (chiL * nuL - chiL * nuLR) + R(0.5) * (rabs(Sal) - nuLR * Sal);
     const R dR = R(0.5) * (chiR * nuR - chiR * nuLR) + R(0.5) * (rabs(Sar) - nuLR * Sar);
     const R aL = R(0.5) * (R(1) + nuLR), aR = R(0.5) * (R(1) - nuLR);
@@ -550,7 +574,8 @@ __device__ __forceinline__ R mhd_hlld_line(const R* vl, const R* vr, R* flux, R 
   }
   {
     const R aR_1 = GP_MAX(R(0), Sr), aL_1 = GP_MIN(R(0), Sl);
-    const R y = ar.inv_pos(aR_1 - aL_1);
+    R y = dS_1;  // the same divisor inside the fan
+    if (!(Sl < R(0) && Sr > R(0))) y = ar.inv_pos(aR_1 - aL_1);
     ct.eb = (aR_1 * vl[VXt] - aL_1 * vr[VXt]) * y;
     ct.et = -(aR_1 * vl[VXb] - aL_1 * vr[VXb]) * y;
     if constexpr (CT != CT_UCT_HLLD) {
@@ -565,27 +590,28 @@ __device__ __forceinline__ R mhd_hlld_line(const R* vl, const R* vr, R* flux, R 
   const bool hllc = ((S1L - Sl) < R(1.e-4) * (SM - Sl)) || ((S1R - Sr) > -R(1.e-4) * (Sr - SM));
   R BtL, BbL, BtR, BbR;
   {
-    const R kL = ar.div(rdl * dul - Bx * Bx, rdl * dsl - Bx * Bx);
-    const R kR = ar.div(rdr * dur - Bx * Bx, rdr * dsr - Bx * Bx);
-    BtL = ul[BXt] * kL;
-    BbL = ul[BXb] * kL;
-    BtR = ur[BXt] * kR;
-    BbR = ur[BXb] * kR;
+    const R kL = ar.div_any(rdl * dul - Bx * Bx, rdl * dsl - Bx * Bx);
+    const R kR = ar.div_any(rdr * dur - Bx * Bx, rdr * dsr - Bx * Bx);
+    BtL = vl[BXt] * kL;
+    BbL = vl[BXb] * kL;
+    BtR = vr[BXt] * kR;
+    BbR = vr[BXb] * kR;
   }
   if (hllc) {
     const R flt = vl[BXt] * vl[VXn] - vl[BXn] * vl[VXt];
     const R frt = vr[BXt] * vr[VXn] - vr[BXn] * vr[VXt];
     const R flb = vl[BXb] * vl[VXn] - vl[BXn] * vl[VXb];
     const R frb = vr[BXb] * vr[VXn] - vr[BXn] * vr[VXb];
-    BtL = BtR = (Sr * ur[BXt] - Sl * ul[BXt] + flt - frt) * dS_1;
-    BbL = BbR = (Sr * ur[BXb] - Sl * ul[BXb] + flb - frb) * dS_1;
+    BtL = BtR = (Sr * vr[BXt] - Sl * vl[BXt] + flt - frt) * dS_1;
+    BbL = BbR = (Sr * vr[BXb] - Sl * vl[BXb] + flb - frb) * dS_1;
     S1L = S1R = SM;
   }
-  const R wL = ar.div(Bx, rdl), wR = ar.div_pos(Bx, rdr);
-  const R vsL = vl[VXt] - wL * (BtL - ul[BXt]);
-  const R vsR = vr[VXt] - wR * (BtR - ur[BXt]);
-  const R wsL = vl[VXb] - wL * (BbL - ul[BXb]);
-  const R wsR = vr[VXb] - wR * (BbR - ur[BXb]);
+  const R wL = ar.quot_bpos(-Bx, -rdl, ar.inv_pos(-rdl));  // rdl < 0 < rdr
+  const R wR = ar.quot_bpos(Bx, rdr, ar.inv_pos(rdr));
+  const R vsL = vl[VXt] - wL * (BtL - vl[BXt]);
+  const R vsR = vr[VXt] - wR * (BtR - vr[BXt]);
+  const R wsL = vl[VXb] - wL * (BbL - vl[BXb]);
+  const R wsR = vr[VXb] - wR * (BbR - vr[BXb]);
 
   // the side and the region: 0 outside the fan, 1 star, 2 double star
   const bool outL = Sl >= R(0), outR = !outL && Sr <= R(0);
@@ -594,13 +620,10 @@ __device__ __forceinline__ R mhd_hlld_line(const R* vl, const R* vr, R* flux, R 
   const bool outside = outL || outR, twice = !(starL || starR);
   R v[8], u[8], f[8];
 #pragma unroll
-  for (int nv = 0; nv < 8; nv++) {
-    v[nv] = left ? vl[nv] : vr[nv];
-    u[nv] = (nv >= BX1 && nv <= BX3) ? v[nv] : (left ? ul[nv] : ur[nv]);
-  }
-  u[RHO] = v[RHO];
+  for (int nv = 0; nv < 8; nv++) v[nv] = left ? vl[nv] : vr[nv];
+  mhd_prim2cons(v, u, gamma - R(1), ygm, ar);
   const R S = left ? Sl : Sr, dv = left ? dul : dur, pt = left ? ptl : ptr;
-  const R ds = left ? dsl : dsr, ys = left ? ysl : ysr, rhos = left ? rhosl : rhosr;
+  const R ds = left ? -dsl : dsr, ys = left ? ysl : ysr, rhos = left ? rhosl : rhosr;
   const R vs = left ? vsL : vsR, ws = left ? wsL : wsR;
   const R Bt = left ? BtL : BtR, Bb = left ? BbL : BbR;
   R us[8];
@@ -614,16 +637,26 @@ __device__ __forceinline__ R mhd_hlld_line(const R* vl, const R* vr, R* flux, R 
   const R vBs = SM * Bx + vs * Bt + ws * Bb;
   scrh = v[VXn] * Bx + v[VXt] * u[BXt] + v[VXb] * u[BXb];
   scrh -= vBs;
-  us[7] = ar.quot(dv * u[7] - pt * v[VXn] + pts * SM + Bx * scrh, ds, ys);
+  R es = dv * u[7] - pt * v[VXn] + pts * SM + Bx * scrh;
+  ar.check(es);
+  us[7] = ar.quot_bpos(left ? -es : es, ds, ys);  // over |S - SM|
   R ptf;
   mhd_flux<DIR>(v, u, f, ptf);
   // double star: common transverse state
   {
-    const R dq = sqrL + sqrR, yq = ar.inv_pos(dq);
-    const R vss = ar.quot(sqrL * vsL + sqrR * vsR + (BtR - BtL) * sBx, dq, yq);
-    const R wss = ar.quot(sqrL * wsL + sqrR * wsR + (BbR - BbL) * sBx, dq, yq);
-    const R Btt = ar.quot(sqrL * BtR + sqrR * BtL + sqrL * sqrR * (vsR - vsL) * sBx, dq, yq);
-    const R Bbb = ar.quot(sqrL * BbR + sqrR * BbL + sqrL * sqrR * (wsR - wsL) * sBx, dq, yq);
+    const R dq = sqrL + sqrR, yq = ar.inv_in(dq);
+    R vss = sqrL * vsL + sqrR * vsR + (BtR - BtL) * sBx;
+    R wss = sqrL * wsL + sqrR * wsR + (BbR - BbL) * sBx;
+    R Btt = sqrL * BtR + sqrR * BtL + sqrL * sqrR * (vsR - vsL) * sBx;
+    R Bbb = sqrL * BbR + sqrR * BbL + sqrL * sqrR * (wsR - wsL) * sBx;
+    ar.check(vss);
+    ar.check(wss);
+    ar.check(Btt);
+    ar.check(Bbb);
+    vss = ar.quot_bpos(vss, dq, yq);
+    wss = ar.quot_bpos(wss, dq, yq);
+    Btt = ar.quot_bpos(Btt, dq, yq);
+    Bbb = ar.quot_bpos(Bbb, dq, yq);
     scrh = vBs;
     scrh -= SM * Bx + vss * Btt + wss * Bbb;
     const R e = (left ? sqrL : sqrR) * scrh * sBx;
@@ -827,8 +860,8 @@ __device__ __forceinline__ R mhd_hlld(const R* vl, const R* vr, R* flux, R gamma
 
 // A face through memory, for the out-of-line solvers: io = vl, vr, gamma, Bn
 // in; flux, face data and cmax out.
-__device__ __forceinline__ void face_in(double* io, const double* vl, const double* vr,
-                                        double gamma, double Bn) {
+template <typename R>
+__device__ __forceinline__ void face_in(R* io, const R* vl, const R* vr, R gamma, R Bn) {
 #pragma unroll
   for (int nv = 0; nv < 8; nv++) {
     io[nv] = vl[nv];
@@ -837,8 +870,8 @@ __device__ __forceinline__ void face_in(double* io, const double* vl, const doub
   io[16] = gamma;
   io[17] = Bn;
 }
-__device__ __forceinline__ void face_out(double* io, const double* flux, const CTFace<double>& ct,
-                                         double cmax) {
+template <typename R>
+__device__ __forceinline__ void face_out(R* io, const R* flux, const CTFace<R>& ct, R cmax) {
 #pragma unroll
   for (int nv = 0; nv < 8; nv++) io[nv] = flux[nv];
   io[8] = ct.eb;
@@ -849,7 +882,8 @@ __device__ __forceinline__ void face_out(double* io, const double* flux, const C
   io[13] = ct.dR;
   io[14] = cmax;
 }
-__device__ __forceinline__ double face_back(const double* io, double* flux, CTFace<double>& ct) {
+template <typename R>
+__device__ __forceinline__ R face_back(const R* io, R* flux, CTFace<R>& ct) {
 #pragma unroll
   for (int nv = 0; nv < 8; nv++) flux[nv] = io[nv];
   ct.eb = io[8];
@@ -862,24 +896,23 @@ __device__ __forceinline__ double face_back(const double* io, double* flux, CTFa
 }
 
 // mhd_hlld out of line, for the few faces mhd_hlld_line hands back
-template <int DIR, int CT>
-__device__ __noinline__ void mhd_hlld_call(double* io) {
-  double flux[8];
-  CTFace<double> ct;
-  const double cmax = mhd_hlld<DIR, CT>(io, io + 8, flux, io[16], io[17], ct);
+template <int DIR, int CT, typename R>
+__device__ __noinline__ void mhd_hlld_call(R* io) {
+  R flux[8];
+  CTFace<R> ct;
+  const R cmax = mhd_hlld<DIR, CT>(io, io + 8, flux, io[16], io[17], ct);
   face_out(io, flux, ct, cmax);
 }
 
-// FP64 HLLD: the straight-line form, and mhd_hlld where its flag is set.
-template <int DIR, int CT>
-__device__ __forceinline__ double mhd_hlld_fp64(const double* vl, const double* vr, double* flux,
-                                                double gamma, double ygm, double Bn,
-                                                CTFace<double>& ct) {
-  FastArith ar;
-  ar.bad = ygm == 0.0;
-  double cmax = mhd_hlld_line<DIR, CT>(vl, vr, flux, gamma, ygm, Bn, ct, ar);
-  if (ar.bad) {
-    double io[18];
+// HLLD of both forms: the straight-line solver, and mhd_hlld where its flag is
+// set.
+template <int DIR, int CT, typename R>
+__device__ __forceinline__ R mhd_hlld_face(const R* vl, const R* vr, R* flux, R gamma, R ygm,
+                                           R Bn, CTFace<R>& ct) {
+  std::conditional_t<sizeof(R) == sizeof(double), FastArith, FloatArith> ar;
+  R cmax = mhd_hlld_line<DIR, CT>(vl, vr, flux, gamma, ygm, Bn, ct, ar);
+  if (ar.bad || ygm == R(0)) {
+    R io[18];
     face_in(io, vl, vr, gamma, Bn);
     mhd_hlld_call<DIR, CT>(io);
     cmax = face_back(io, flux, ct);
@@ -1154,7 +1187,7 @@ __device__ __forceinline__ R hd_hllc_line(const R* vl, const R* vr, R* flux, R g
     const R qL = vl[4] + vl[RHO] * vl[VXn] * (vl[VXn] - Sl);
     const R qR = vr[4] + vr[RHO] * vr[VXn] * (vr[VXn] - Sr);
     const R wL = vl[RHO] * (vl[VXn] - Sl), wR = vr[RHO] * (vr[VXn] - Sr);
-    vs = ar.div(qR - qL, wR - wL);
+    vs = ar.div_any(qR - qL, wR - wL);
   }
   const bool outL = Sl > R(0), outR = !outL && Sr < R(0);
   const bool left = outL || (!outR && vs >= R(0));
@@ -1168,14 +1201,16 @@ __device__ __forceinline__ R hd_hllc_line(const R* vl, const R* vr, R* flux, R g
   u[MX3] = v[RHO] * v[VX1 + 2];
   R kin = v[VX1] * v[VX1] + v[VX1 + 1] * v[VX1 + 1] + v[VX1 + 2] * v[VX1 + 2];
   kin = v[RHO] * kin * R(0.5);
-  u[4] = kin + ar.quot_pos(v[4], gamma - R(1), ygm);
+  u[4] = kin + ar.quot_bpos(v[4], gamma - R(1), ygm);
   hd_flux<DIR>(v, u, f, p);
   const R vx = v[VXn];
-  us[RHO] = ar.div(u[RHO] * (S - vx), S - vs);
+  us[RHO] = ar.div_any(u[RHO] * (S - vx), S - vs);
   us[MXn] = us[RHO] * vs;
   us[MXt] = us[RHO] * v[VXt];
   us[MXb] = us[RHO] * v[VXb];
-  us[4] = ar.quot(u[4], v[RHO], y) + (vs - vx) * (vs + ar.div(v[4], v[RHO] * (S - vx)));
+  ar.check(u[4]);
+  us[4] = ar.quot_bpos(u[4], v[RHO], y) +
+          (vs - vx) * (vs + ar.div_any(v[4], v[RHO] * (S - vx)));
   us[4] *= us[RHO];
 #pragma unroll
   for (int nv = 0; nv < 5; nv++) {
