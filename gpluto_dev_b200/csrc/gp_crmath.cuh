@@ -19,8 +19,8 @@
 //    series (double-double through the r^7 / r^6 terms, double beyond), then
 //    the addition formulas with sin(j/16), cos(j/16) held as double-double
 //    constants (computed to 300 bits).  Relative error about 2^-100.
-//  * acos_cr(x), -1 <= x <= 1: one Newton step on sin(y) = s from the
-//    library's asin (a few ulps), with s = x for |x| <= 1/2
+//  * acos_cr(x), -1 <= x <= 1 (full-accuracy path): one Newton step on sin(y) = s
+//    from the library's asin (a few ulps), with s = x for |x| <= 1/2
 //    (acos = pi/2 - asin x) and s = sqrt((1 -+ x)/2) as a double-double
 //    otherwise (acos = 2 asin s, or pi - 2 asin s; 1 -+ x is exact there).
 //    Newton's error is quadratic in the start error, ~2^-100 relative.
@@ -37,6 +37,7 @@
 #include <math.h>
 
 #if defined(__CUDACC__)
+#include "gp_exact.cuh"
 #define GP_CR_FN __host__ __device__ __forceinline__
 #define GP_CR_SLOW static __host__ __device__ __noinline__
 #else
@@ -338,9 +339,31 @@ GP_CR_FN void sincos_cr(double x, double* sn, double* cs) {
   if (!ok) sincos_slow(x, sn, cs);
 }
 
-// correctly rounded acos(x), -1 <= x <= 1: the Newton step of asin_dd on the
-// fast sin (its error carried through: |d asin / d sin| = 1/cos <= 1.16 on
-// [-1/2, 1/2], doubled where acos = 2 asin), then the rounding test.
+// 1/x and sqrt(t) for arguments of order one: straight-line on the device
+GP_CR_FN double inv_cr(double x) {
+#if defined(__CUDA_ARCH__)
+  return gp::FastArith().inv_in(x);
+#else
+  return 1.0 / x;
+#endif
+}
+GP_CR_FN double sqrt_cr(double t) {
+#if defined(__CUDA_ARCH__)
+  return gp::FastArith().root0(t);
+#else
+  return sqrt(t);
+#endif
+}
+
+// correctly rounded acos(x), -1 <= x <= 1.  asin(s) starts from the FP32
+// function (the FP64 one took a third of this function's time), y0 within
+// 2^-21 of it relative, and takes the inverse sine's Taylor step to third
+// order in d = (s - sin y0) / cos y0:
+//   asin s = y0 + d + t/2 d^2 + (1 + 3 t^2)/6 d^3 + O(d^4),  t = tan y0,
+// the neglected term below 2^-83 relative and the step's own roundings below
+// 2^-71 relative; the error of the fast sin is carried through (|d asin / d
+// sin| = 1/cos <= 1.16 on [-1/2, 1/2], doubled where acos = 2 asin).  Then the
+// rounding test.
 GP_CR_FN double acos_cr(double x) {
   const double kPih = 0x1.921fb54442d18p+1, kPil = 0x1.1a62633145c07p-53;
   const double kPi2h = 0x1.921fb54442d18p+0, kPi2l = 0x1.1a62633145c07p-54;
@@ -351,19 +374,21 @@ GP_CR_FN double acos_cr(double x) {
     sl = 0.0;
   } else {
     const double t = (x > 0.0 ? 1.0 - x : 1.0 + x) * 0.5;   // exact
-    sh = sqrt(t);
-    sl = sh > 0.0 ? fma(-sh, sh, t) / (2.0 * sh) : 0.0;
+    sh = sqrt_cr(t);
+    sl = fma(-sh, sh, t) * (0.5 * inv_cr(sh > 0.0 ? sh : 1.0));
   }
-  const double y0 = asin(sh);
+  const double y0 = (double)asinf((float)sh);
   dd sy;
   double es, cy;
   sin_fast_cos_d(fabs(y0), sy, es, cy);
   if (y0 < 0.0) sy = dd_neg(sy);
-  // s - sin(y0): the high parts are within a few ulps (exact difference)
+  // s - sin(y0): the high parts are within a factor of 2 (exact difference)
   const double e = (sh - sy.hi) + (sl - sy.lo);
-  const double delta = e / cy;
+  const double ic = inv_cr(cy);
+  const double d = e * ic, tn = sy.hi * ic;
+  const double delta = fma(d * d, fma(d, fma(tn, tn, 1.0 / 3.0) * 0.5, 0.5 * tn), d);
   dd y;
-  double err = 1.25 * es;
+  double err = fma(0x1p-69, fabs(y0), 1.25 * es);
   if (mid) {
     const dd t = two_sum(kPi2h, -y0);
     y = fast_two_sum(t.hi, (t.lo - delta) + kPi2l);
@@ -375,8 +400,6 @@ GP_CR_FN double acos_cr(double x) {
     y = fast_two_sum(t.hi, (t.lo - 2.0 * delta) + kPil);
     err *= 2.0;
   }
-  // + the Newton step's own terms (quadratic in a few ulps, relative)
-  err += 0x1p-98 * fabs(y.hi);
   double r;
   if (round_certain(y, err, &r)) return r;
   return acos_slow(x);
