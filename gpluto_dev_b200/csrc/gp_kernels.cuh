@@ -113,6 +113,16 @@ __device__ __forceinline__ void cp_async_wait0() {
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
+// Programmatic dependent launch: a kernel of the step lets the next one's
+// blocks be placed as soon as all of its own are running, and touches memory
+// only after every kernel before it has completed.  Small grids are bound by
+// the launches' latency (2-D MHD 64^2: step 82 -> 72 us; 256^2, ten steps: 808
+// -> 704 us).
+__device__ __forceinline__ void step_order() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 #ifndef GP_SWEEP_MINB
 #define GP_SWEEP_MINB 3
 #endif
@@ -813,6 +823,7 @@ template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, typename R, typen
 __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_x_minb<PHYS, R>()))
     sweep_x_kernel(StageArgs<CTT> a, Grid3 g, int nseg) {
   __shared__ double stg[sweep_x_stage_doubles<NV, LIM>()];
+  step_order();
   const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int row = w / nseg, q = w - row * nseg;
   sweep_x_row<PHYS, NV, NDIM, RS, CT, LIM, R, CTT>(a, g, row, (int)((long long)g.nx * q / nseg),
@@ -1156,6 +1167,7 @@ template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, typename
 __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_m_minb<PHYS, R>()))
     sweep_m_kernel(StageArgs<CTT> a, Grid3 g, int S, bool flat) {
   __shared__ double stg[sweep_m_stage_doubles<NV, LIM>()];
+  step_order();
   const int nd = (DIR == 1) ? g.ny : g.nz;
   const int nseg = (nd + S - 1) / S;
   int i, t, seg;
@@ -1344,6 +1356,7 @@ __device__ __forceinline__ void emf_cell(const StageArgs<CTT>& a, const Grid3& g
 
 template <int NDIM, int LIM, typename R, typename CTT>
 __global__ void __launch_bounds__(256, 4) emf_kernel(StageArgs<CTT> a, Grid3 g) {
+  step_order();
   emf_cell<NDIM, LIM, R, CTT>(a, g, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -1374,6 +1387,7 @@ __device__ __forceinline__ void coef_pair(const R* f1, const R* f2, R& aL, R& aR
 template <int LIM, typename R, typename CTT>
 __global__ void __launch_bounds__(EMF_TX * EMF_TY, 3)
     emf_march_kernel(StageArgs<CTT> a, Grid3 g, int sz) {
+  step_order();
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int i = blockIdx.x * EMF_TX + threadIdx.x;
   const int j = blockIdx.y * EMF_TY + threadIdx.y;
@@ -1501,6 +1515,7 @@ __global__ void __launch_bounds__(EMF_TX * EMF_TY, 3)
 // components stored as ct[d][0] = e[b][d], ct[d][1] = e[t][d].
 template <int NDIM, typename R, typename CTT>
 __global__ void __launch_bounds__(256) emf_arith_kernel(StageArgs<CTT> a, Grid3 g) {
+  step_order();
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= g.n) return;
   const int nx = g.nx, ny = g.ny, nz = g.nz, nxy = nx * ny;
@@ -1530,6 +1545,7 @@ __global__ void __launch_bounds__(256) emf_arith_kernel(StageArgs<CTT> a, Grid3 
 // operation order.  Thread per cell, its three edges.
 template <int NDIM, typename R, typename CTT>
 __global__ void __launch_bounds__(256) emf_contact_kernel(StageArgs<CTT> a, Grid3 g) {
+  step_order();
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= g.n) return;
   const int nx = g.nx, ny = g.ny, nz = g.nz, nxy = nx * ny;
@@ -1693,6 +1709,7 @@ __device__ __forceinline__ void coef_tile(const CTT* k, int n, int e, R* c) {
 template <int LIM, typename R, typename CTT>
 __global__ void __launch_bounds__(ET_THREADS, (emf_tile_minb<R>()))
     emf_tile_kernel(StageArgs<CTT> a, Grid3 g, int sz) {
+  step_order();
   using T = EmfTile<LIM, CTT>;
   constexpr int W = T::W, HL = T::HL, HR = W - 1 - HL, XW = T::XW, YH = T::YH;
   extern __shared__ __align__(16) unsigned char emf_smem[];
@@ -1991,6 +2008,7 @@ __host__ __device__ constexpr int finish_minb() { return sizeof(CTT) == 4 ? 6 : 
 
 template <int PHYS, int NV, int NDIM, typename CTT>
 __global__ void __launch_bounds__(256, finish_minb<CTT>()) finish_kernel(StageArgs<CTT> a, Grid3 g) {
+  step_order();
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const double cdt = finish_cell<PHYS, NV, NDIM, CTT>(a, g, c);
   // per-warp maximum: a block-wide one (a barrier per block) made the FP64

@@ -68,6 +68,22 @@ static StageArgs<CTT> make_args(const StageDesc& d) {
   return a;
 }
 
+// Launch in stream order, the next launch's blocks placed early (step_order)
+template <typename... K, typename... A>
+static void launch(void (*k)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute early;
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &early;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, k, K(args)...);
+}
+
 // Parts an x-row is swept in.  A warp solves 32 faces at a time and a part
 // one face more than its cells, so k chunks hold 32 k - 1 cells; a whole
 // periodic row needs no extra face.  The count with the fewest (waves of
@@ -126,7 +142,7 @@ static void launch_m(const StageArgs<CTT>& a, const Grid3& g, int nt, int nd, cu
   pre();
   const bool flat = g.nx % SWEEP_THREADS != 0 || (long long)nt * nseg > 65535;
   const dim3 grid = flat ? dim3((unsigned)(cols * nseg)) : dim3(g.nx / SWEEP_THREADS, nt * nseg);
-  sweep_m_kernel<PHYS, NV, NDIM, RS, CT, LIM, DIR, RT, CTT><<<grid, SWEEP_THREADS, 0, s>>>(a, g, seg, flat);
+  launch(sweep_m_kernel<PHYS, NV, NDIM, RS, CT, LIM, DIR, RT, CTT>, grid, SWEEP_THREADS, 0, s, a, g, seg, flat);
   post();
 }
 
@@ -149,7 +165,7 @@ static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, cudaStream_t 
     const int nseg = x_segments<PHYS, LIM, RT>(gd.nx, rows);
     dim3 grid((unsigned)(((long long)rows * nseg + wpb - 1) / wpb));
     pre();
-    sweep_x_kernel<PHYS, NV, NDIM, RS, CT, LIM, RT, CTT><<<grid, SWEEP_THREADS, 0, s>>>(a, g, nseg);
+    launch(sweep_x_kernel<PHYS, NV, NDIM, RS, CT, LIM, RT, CTT>, grid, SWEEP_THREADS, 0, s, a, g, nseg);
     post();
   }
   launch_m<PHYS, NV, NDIM, RS, CT, LIM, 1>(a, g, gd.nz, gd.ny, s, pre, post);
@@ -159,9 +175,9 @@ static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, cudaStream_t 
   if constexpr (PHYS != PHYS_HD) {
     pre();
     if constexpr (CT == CT_ARITH) {
-      emf_arith_kernel<NDIM, RT, CTT><<<nb, 256, 0, s>>>(a, g);
+      launch(emf_arith_kernel<NDIM, RT, CTT>, nb, 256, 0, s, a, g);
     } else if constexpr (CT == CT_CONTACT) {
-      emf_contact_kernel<NDIM, RT, CTT><<<nb, 256, 0, s>>>(a, g);
+      launch(emf_contact_kernel<NDIM, RT, CTT>, nb, 256, 0, s, a, g);
     } else if constexpr (NDIM == 3 && (sizeof(RT) == 8 || five_point<LIM>())) {  // plane-staged EMF
       using T = EmfTile<LIM, CTT>;
       cudaFuncSetAttribute(emf_tile_kernel<LIM, RT, CTT>,
@@ -172,7 +188,7 @@ static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, cudaStream_t 
       int sz = ET_SEGMENT;
       while (sz > 4 && cols * ((gd.nz + sz - 1) / sz) < 148LL * emf_tile_minb<RT>() * 4) sz /= 2;
       dim3 grid((gd.nx + ETX - 1) / ETX, (gd.ny + ETY - 1) / ETY, (gd.nz + sz - 1) / sz);
-      emf_tile_kernel<LIM, RT, CTT><<<grid, dim3(ETX, ETY), T::SMEM, s>>>(a, g, sz);
+      launch(emf_tile_kernel<LIM, RT, CTT>, grid, dim3(ETX, ETY), T::SMEM, s, a, g, sz);
     } else if constexpr (NDIM == 3) {  // mixed PLM/PPM: z-marching EMF, loads through L1
       // the longest segment (<= EMF_SEGMENT planes) that still gives about
       // four waves of blocks over 148 SMs (3 blocks per SM)
@@ -182,14 +198,14 @@ static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, cudaStream_t 
       while (sz > 4 && cols * ((gd.nz + sz - 1) / sz) < 148LL * 3 * 4) sz /= 2;
       dim3 grid((gd.nx + EMF_TX - 1) / EMF_TX, (gd.ny + EMF_TY - 1) / EMF_TY,
                 (gd.nz + sz - 1) / sz);
-      emf_march_kernel<LIM, RT, CTT><<<grid, dim3(EMF_TX, EMF_TY), 0, s>>>(a, g, sz);
+      launch(emf_march_kernel<LIM, RT, CTT>, grid, dim3(EMF_TX, EMF_TY), 0, s, a, g, sz);
     } else {
-      emf_kernel<NDIM, LIM, RT, CTT><<<nb, 256, 0, s>>>(a, g);
+      launch(emf_kernel<NDIM, LIM, RT, CTT>, nb, 256, 0, s, a, g);
     }
     post();
   }
   pre();
-  finish_kernel<PHYS, NV, NDIM, CTT><<<nb, 256, 0, s>>>(a, g);
+  launch(finish_kernel<PHYS, NV, NDIM, CTT>, nb, 256, 0, s, a, g);
   post();
 }
 
