@@ -776,8 +776,10 @@ int gp_create(const gp_grid_desc* grid, const gp_scheme* scheme, void* stream,
   alloc((void**)&h->V, cell * h->nvar);
   // flux differences, inverse-dt terms, UCT data and EMFs: float in the mixed form
   const size_t fcell = (h->mixed ? sizeof(float) : sizeof(double)) * h->pn;
-  alloc((void**)&h->dU, fcell * h->nvar * 3);
-  alloc((void**)&h->Cdt, fcell * 3);
+  // one array per direction, or their sum (gp::sum_directions)
+  const int ndu = scheme->physics == GP_HD && !h->mixed ? 1 : 3;
+  alloc((void**)&h->dU, fcell * h->nvar * ndu);
+  alloc((void**)&h->Cdt, fcell * ndu);
   if (scheme->physics != GP_HD) {
     for (int b = 0; b < 3; b++)
       for (int d = 0; d < h->ndim; d++) alloc((void**)&h->Bs[b][d], cell);
@@ -796,8 +798,8 @@ int gp_create(const gp_grid_desc* grid, const gp_scheme* scheme, void* stream,
     return fail(GP_ERR_NOMEM, "device allocation failed for %lld cells", ncell);
   }
   cudaMemsetAsync(h->sc, 0, sizeof(StepScalars), h->stream);
-  cudaMemsetAsync(h->dU, 0, fcell * h->nvar * 3, h->stream);
-  cudaMemsetAsync(h->Cdt, 0, fcell * 3, h->stream);
+  cudaMemsetAsync(h->dU, 0, fcell * h->nvar * ndu, h->stream);
+  cudaMemsetAsync(h->Cdt, 0, fcell * ndu, h->stream);
   h->bcur = 0;
   {
     int fills = 0;

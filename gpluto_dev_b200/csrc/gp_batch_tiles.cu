@@ -53,7 +53,7 @@ __device__ __forceinline__ void sweep_m_item(const StageArgs<CTT>& a, const Grid
   const long long r = item / g.nx;
   const int seg = (int)(r % nseg);
   const int t = (int)(r / nseg);
-  sweep_m_col<PHYS, NV, NDIM, RS, CT, LIM, DIR, RT, CTT>(a, g, i, t, seg, S, smem, tid);
+  sweep_m_col<PHYS, NV, NDIM, RS, CT, LIM, DIR, false, RT, CTT>(a, g, i, t, seg, S, smem, tid);
 }
 
 // One non-inlined function per (scheme, phase): each gets its own register
@@ -87,7 +87,7 @@ __device__ __noinline__ void tile_finish(const StageArgs<CTT>& a, Grid3 g, int c
   const long long c0 = (long long)idx * BATCH_THREADS * cpt + threadIdx.x;
   double mx = 0.0;
   for (int q = 0; q < cpt; q++) {
-    const double cdt = finish_cell<PHYS, NV, NDIM, CTT>(a, g, c0 + (long long)q * BATCH_THREADS);
+    const double cdt = finish_cell<PHYS, NV, NDIM, false, CTT>(a, g, c0 + (long long)q * BATCH_THREADS);
     mx = GP_MAX(mx, cdt);
   }
   if (stage == 1) warp_invdt_max(a.invdt_bits, mx, threadIdx.x & 31);

@@ -57,8 +57,8 @@ struct StageArgs {
   const double* Bs[3];    // stage-input face fields (left faces)
   const double* Bs0[3];   // face fields at t^n (stage 2)
   double* Bsout[3];       // face fields written by this stage
-  CTT* dU;                // [3][nvar][n] flux difference of each direction
-  CTT* Cdt;               // [3][n] inverse dt of each direction
+  CTT* dU;                // [3][nvar][n] flux difference of each direction, or [nvar][n] their sum
+  CTT* Cdt;               // [3][n] inverse dt of each direction, or [n] their sum
   const double* U0;       // U^n
   const double* Uc;       // stage-input U
   double* Uout;           // U written by this stage
@@ -144,6 +144,15 @@ constexpr int sweep_m_minb() {
   return PHYS == PHYS_RMHD ? (sizeof(R) == 4 ? 3 : 2) : (sizeof(R) == 4 ? 5 : 4);
 }
 
+// whether the single-grid kernels add the directions' flux differences up in
+// one array (see cell_update): the FP64 form of hydrodynamics (160^3: finish
+// 164 -> 114 us, y and z sweeps 98 -> 107 each).  For MHD the sweeps lost what
+// the finish gained (256^3: 971 -> 859 against 926 -> 966 twice).
+template <int PHYS, typename CTT>
+__host__ __device__ constexpr bool sum_directions() {
+  return PHYS == PHYS_HD && sizeof(CTT) == sizeof(double);
+}
+
 // whether conserved component nv receives a flux difference that survives
 // the stage (the cell-centred field along active directions is overwritten
 // by the face average, Src/MHD/CT/ct_field_average.cpp:378-410)
@@ -208,23 +217,31 @@ __device__ __forceinline__ R riemann(const R* vl, const R* vr, R* flux, R gamma,
 // 981) and its inverse-dt term (Src/MHD/rhs.cpp:523 and the += at 756, 981),
 // written to the direction's own arrays; the finish kernel sums them in the
 // order x, y, z as Src/update_stage.cpp:173-184/272-284/369-380 does.
+//
+// With `sum` (sum_directions) there is one array for all
+// directions: the x-sweep writes it and the y and z sweeps add to it, in that
+// order, sum[0 .. NV] being what the cell held.  The sweeps are bound by
+// arithmetic, the finish by HBM, which reads 96 bytes a cell less that way
+// (3-D).
 template <int PHYS, int NV, int NDIM, typename R, typename CTT>
 __device__ __forceinline__ void cell_update(const StageArgs<CTT>& a, long long n,
                                             long long c, const R* Fl, const R* Fr,
-                                            R cml, R cmr, int dir) {
-  CTT* du = a.dU + (long long)dir * NV * n;
+                                            R cml, R cmr, int dir, const R* sum = nullptr) {
+  CTT* du = a.dU + (sum ? 0 : (long long)dir * NV * n);
   if constexpr (sizeof(R) == sizeof(double)) {
     const double dtdx = a.dtdx[dir];
 #pragma unroll
     for (int nv = 0; nv < NV; nv++) {
       if (!rhs_var<PHYS, NDIM>(nv)) continue;
-      du[nv * n + c] = (CTT)(-dtdx * ((double)Fr[nv] - (double)Fl[nv]));
+      const double r = -dtdx * ((double)Fr[nv] - (double)Fl[nv]);
+      du[nv * n + c] = (CTT)(sum ? (double)sum[nv] + r : r);
     }
     // stored in every stage although only stage 1's CFL maximum reads it
     // (Src/update_stage.cpp:422-435): a store conditional on the stage made
     // the FP64 y/z sweeps 40% slower at 256^3
-    a.Cdt[(long long)dir * n + c] =
-        (CTT)fixed_quot(0.5 * ((double)cml + (double)cmr), a.dx[dir], a.inv_dx[dir]);
+    const double q = fixed_quot(0.5 * ((double)cml + (double)cmr), a.dx[dir], a.inv_dx[dir]);
+    if (sum) a.Cdt[c] = (CTT)((double)sum[NV] + q);
+    else a.Cdt[(long long)dir * n + c] = (CTT)q;
   } else {
     // mixed form: the stored difference is FP32, so it is formed in FP32
     // (no widening and narrowing conversions, no FP64 division)
@@ -280,9 +297,15 @@ constexpr int sweep_x_stage_doubles() {
 }
 // y/z sweeps: a ring of four cells and two face fields per thread (PLM,
 // LimO3, WENO3), two cells and face fields otherwise
-template <int NV, int LIM = LIM_MC>
+// values SumStage keeps of a cell: flux differences (at most 6 with a field in
+// two directions) and the inverse-dt term
+template <int NV>
+constexpr int sum_slots() { return NV == 8 ? 7 : NV + 1; }
+template <int NV, int LIM = LIM_MC, bool SUM = false>
 constexpr int sweep_m_stage_doubles() {
-  return ((LIM == LIM_PPM || five_point<LIM>()) ? 2 * (NV + 1) : 4 * NV + 2) * SWEEP_THREADS;
+  return (((LIM == LIM_PPM || five_point<LIM>()) ? 2 * (NV + 1) : 4 * NV + 2) +
+          (SUM ? 2 * sum_slots<NV>() : 0)) *
+         SWEEP_THREADS;
 }
 
 // Piecewise parabolic x-row (one warp per row).  Lane l of a chunk owns
@@ -838,11 +861,48 @@ __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_x_minb<PHYS, R>()))
 // is solved.  Writes the direction's flux differences, inverse-dt terms and
 // UCT face data (no loads besides the stencil).
 // ---------------------------------------------------------------------
+// The flux differences and inverse-dt term the directions before left in a
+// cell, staged into shared memory an iteration before they are added to
+// (two slots per thread).
+template <int PHYS, int NV, int NDIM, bool SUM, typename CTT>
+struct SumStage {
+  const StageArgs<CTT>& a;
+  long long n;
+  double* s;
+  int tid;
+  static constexpr int K = sum_slots<NV>();
+  // slot of component nv (NV: the inverse-dt term), without the unused field ones
+  static constexpr __device__ int at(int nv) {
+    return (PHYS != PHYS_HD && nv >= BX1) ? nv - NDIM : nv;
+  }
+  __device__ __forceinline__ void load(long long c, int slot) {
+    if constexpr (SUM) {
+      double* d = s + slot * K * SWEEP_THREADS + tid;
+#pragma unroll
+      for (int nv = 0; nv < NV; nv++)
+        if (rhs_var<PHYS, NDIM>(nv)) cp_async8(d + at(nv) * SWEEP_THREADS, a.dU + nv * n + c);
+      cp_async8(d + at(NV) * SWEEP_THREADS, a.Cdt + c);
+    }
+  }
+  template <typename R>
+  __device__ __forceinline__ const R* get(int slot, R* v) {
+    if constexpr (SUM) {
+      const double* d = s + slot * K * SWEEP_THREADS + tid;
+#pragma unroll
+      for (int nv = 0; nv <= NV; nv++)
+        if (nv == NV || rhs_var<PHYS, NDIM>(nv)) v[nv] = d[at(nv) * SWEEP_THREADS];
+      return v;
+    }
+    return nullptr;
+  }
+};
+
 // Piecewise parabolic y/z march: cells m-1, m, m+1 in registers, cell m+2
 // staged with cp.async (one iteration ahead: cell m+3 and face m+1 are
 // prefetched while face m is solved).  The constrained value of face m+1 is
 // formed from cells m-1..m+2 and carried to the next iteration as face m's.
-template <int PHYS, int NV, int NDIM, int RS, int CT, int DIR, typename R, typename CTT>
+template <int PHYS, int NV, int NDIM, int RS, int CT, int DIR, bool SUM, typename R,
+          typename CTT>
 __device__ __forceinline__ void sweep_m_col_ppm(const StageArgs<CTT>& a, const Grid3& g, int i,
                                                 int t, int seg, int S, double* stg_, int tid) {
   double(*stg)[NV + 1][SWEEP_THREADS] = reinterpret_cast<double(*)[NV + 1][SWEEP_THREADS]>(stg_);
@@ -864,6 +924,7 @@ __device__ __forceinline__ void sweep_m_col_ppm(const StageArgs<CTT>& a, const G
         cp_async8(&stg[b][NV][tid], a.Bs[DIR] + base + (long long)gidx(mface, nd, g.outflow, DIR) * stride);
       cp_async_commit();
     };
+    SumStage<PHYS, NV, NDIM, SUM, CTT> ss{a, n, stg_ + 2 * (NV + 1) * SWEEP_THREADS, tid};
     stage(m0 + 2, m0, 0);
     R W0[NV], W1[NV], W2[NV], Fm[NV], vLn[NV], Fp[NV], cmp = R(0);
     {
@@ -888,6 +949,7 @@ __device__ __forceinline__ void sweep_m_col_ppm(const StageArgs<CTT>& a, const G
     }
     int buf = 0;
     for (int m = m0; m <= m1; m++, buf ^= 1) {
+      if (m < m1) ss.load(base + (long long)m * stride, m & 1);
       stage(m + 3, m + 1, buf ^ 1);   // prefetch for the next iteration
       cp_async_wait1();
       R vL[NV], vR[NV], F[NV], W3[NV];
@@ -919,9 +981,11 @@ __device__ __forceinline__ void sweep_m_col_ppm(const StageArgs<CTT>& a, const G
       if constexpr (PHYS != PHYS_HD) {
         if (m < m1) store_ct<CT>(a, DIR, base + (long long)gidx(m, nd, g.outflow, DIR) * stride, ct);
       }
-      if (m > m0)
+      if (m > m0) {
+        R sum[NV + 1];
         cell_update<PHYS, NV, NDIM>(a, n, base + (long long)(m - 1) * stride, Fp, F, cmp, cm,
-                                    DIR);
+                                    DIR, ss.get((m - 1) & 1, sum));
+      }
 #pragma unroll
       for (int nv = 0; nv < NV; nv++) {
         W0[nv] = W1[nv];
@@ -936,7 +1000,7 @@ __device__ __forceinline__ void sweep_m_col_ppm(const StageArgs<CTT>& a, const G
   if (err) atomicOr(a.err, err);
 }
 
-template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, typename R,
+template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, bool SUM, typename R,
           typename CTT>
 __device__ __forceinline__ void sweep_m_col_mp5(const StageArgs<CTT>& a, const Grid3& g, int i,
                                                 int t, int seg, int S, double* stg_, int tid) {
@@ -959,6 +1023,7 @@ __device__ __forceinline__ void sweep_m_col_mp5(const StageArgs<CTT>& a, const G
         cp_async8(&stg[b][NV][tid], a.Bs[DIR] + base + (long long)gidx(mface, nd, g.outflow, DIR) * stride);
       cp_async_commit();
     };
+    SumStage<PHYS, NV, NDIM, SUM, CTT> ss{a, n, stg_ + 2 * (NV + 1) * SWEEP_THREADS, tid};
     stage(m0 + 2, m0, 0);
     // window: Wm = cell m-2, W0 = m-1, W1 = m, W2 = m+1, W3 = m+2
     R Wm[NV], W0[NV], W1[NV], W2[NV], vLn[NV], Fp[NV], cmp = R(0);
@@ -981,6 +1046,7 @@ __device__ __forceinline__ void sweep_m_col_mp5(const StageArgs<CTT>& a, const G
     }
     int buf = 0;
     for (int m = m0; m <= m1; m++, buf ^= 1) {
+      if (m < m1) ss.load(base + (long long)m * stride, m & 1);
       stage(m + 3, m + 1, buf ^ 1);   // prefetch for the next iteration
       cp_async_wait1();
       R vL[NV], vR[NV], F[NV], W3[NV];
@@ -1011,9 +1077,11 @@ __device__ __forceinline__ void sweep_m_col_mp5(const StageArgs<CTT>& a, const G
       if constexpr (PHYS != PHYS_HD) {
         if (m < m1) store_ct<CT>(a, DIR, base + (long long)gidx(m, nd, g.outflow, DIR) * stride, ct);
       }
-      if (m > m0)
+      if (m > m0) {
+        R sum[NV + 1];
         cell_update<PHYS, NV, NDIM>(a, n, base + (long long)(m - 1) * stride, Fp, F, cmp, cm,
-                                    DIR);
+                                    DIR, ss.get((m - 1) & 1, sum));
+      }
 #pragma unroll
       for (int nv = 0; nv < NV; nv++) {
         Wm[nv] = W0[nv];
@@ -1032,16 +1100,17 @@ __device__ __forceinline__ void sweep_m_col_mp5(const StageArgs<CTT>& a, const G
 // One (x column i, transverse index t, pencil segment seg) per thread: t is
 // k for DIR=1 and j for DIR=2; the segment covers cells [seg*S, seg*S+S).
 // `stg_` is the block's staging area (sweep_m_stage_doubles<NV>() doubles).
-template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, typename R,
+template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, bool SUM, typename R,
           typename CTT>
 __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3& g, int i, int t,
                                             int seg, int S, double* stg_, int tid) {
   if constexpr (LIM == LIM_PPM) {
-    sweep_m_col_ppm<PHYS, NV, NDIM, RS, CT, DIR, R, CTT>(a, g, i, t, seg, S, stg_, tid);
+    sweep_m_col_ppm<PHYS, NV, NDIM, RS, CT, DIR, SUM, R, CTT>(a, g, i, t, seg, S, stg_, tid);
     return;
   }
   if constexpr (five_point<LIM>()) {
-    sweep_m_col_mp5<PHYS, NV, NDIM, RS, CT, LIM, DIR, R, CTT>(a, g, i, t, seg, S, stg_, tid);
+    sweep_m_col_mp5<PHYS, NV, NDIM, RS, CT, LIM, DIR, SUM, R, CTT>(a, g, i, t, seg, S, stg_,
+                                                                      tid);
     return;
   }
   // Ring of four cells (cell m in slot m & 3) and of two face fields: a
@@ -1076,6 +1145,7 @@ __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3
 #pragma unroll
       for (int nv = 0; nv < NV; nv++) v[nv] = (R)sv[m & 3][nv][tid];
     };
+    SumStage<PHYS, NV, NDIM, SUM, CTT> ss{a, n, stg_ + (4 * NV + 2) * SWEEP_THREADS, tid};
     stage_cell(m0 - 1);
     stage_cell(m0);
     cp_async_commit();
@@ -1106,6 +1176,7 @@ __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3
       if (m < m1) {   // prefetch for the next iteration
         stage_cell(m + 2);
         stage_face(m + 1);
+        ss.load(base + (long long)m * stride, m & 1);
       }
       cp_async_commit();
       cp_async_wait1();
@@ -1145,9 +1216,11 @@ __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3
       if constexpr (PHYS != PHYS_HD) {
         if (m < m1) store_ct<CT>(a, DIR, base + (long long)gidx(m, nd, g.outflow, DIR) * stride, ct);
       }
-      if (m > m0)
+      if (m > m0) {
+        R sum[NV + 1];
         cell_update<PHYS, NV, NDIM>(a, n, base + (long long)(m - 1) * stride, Fp, F, cmp, cm,
-                                    DIR);
+                                    DIR, ss.get((m - 1) & 1, sum));
+      }
 #pragma unroll
       for (int nv = 0; nv < NV; nv++) Fp[nv] = F[nv];
       cmp = cm;
@@ -1166,7 +1239,8 @@ __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3
 template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, typename R, typename CTT>
 __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_m_minb<PHYS, R>()))
     sweep_m_kernel(StageArgs<CTT> a, Grid3 g, int S, bool flat) {
-  __shared__ double stg[sweep_m_stage_doubles<NV, LIM>()];
+  constexpr bool SUM = sum_directions<PHYS, CTT>();
+  __shared__ double stg[sweep_m_stage_doubles<NV, LIM, SUM>()];
   step_order();
   const int nd = (DIR == 1) ? g.ny : g.nz;
   const int nseg = (nd + S - 1) / S;
@@ -1184,7 +1258,8 @@ __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_m_minb<PHYS, R>()))
     t = blockIdx.y / nseg;
     seg = blockIdx.y - t * nseg;
   }
-  sweep_m_col<PHYS, NV, NDIM, RS, CT, LIM, DIR, R, CTT>(a, g, i, t, seg, S, stg, threadIdx.x);
+  sweep_m_col<PHYS, NV, NDIM, RS, CT, LIM, DIR, SUM, R, CTT>(a, g, i, t, seg, S, stg,
+                                                             threadIdx.x);
 }
 
 // ---------------------------------------------------------------------
@@ -1891,7 +1966,7 @@ __device__ __forceinline__ double face_new(const StageArgs<CTT>& a, int d, long 
 }
 
 // Stage finish of cell c; returns its inverse-dt sum (0 outside the grid).
-template <int PHYS, int NV, int NDIM, typename CTT>
+template <int PHYS, int NV, int NDIM, bool SUM, typename CTT>
 __device__ __forceinline__ double finish_cell(const StageArgs<CTT>& a, const Grid3& g,
                                               long long c) {
   const long long n = g.n;
@@ -1903,15 +1978,17 @@ __device__ __forceinline__ double finish_cell(const StageArgs<CTT>& a, const Gri
 #pragma unroll
     for (int nv = 0; nv < NV; nv++) {
       if (!rhs_var<PHYS, NDIM>(nv)) continue;
-      double Rc = (double)a.dU[nv * n + c] + (double)a.dU[(NV + nv) * n + c];
-      if (NDIM == 3) Rc = Rc + (double)a.dU[(2 * NV + nv) * n + c];
+      double Rc = (double)a.dU[nv * n + c];
+      if (!SUM) Rc = Rc + (double)a.dU[(NV + nv) * n + c];
+      if (!SUM && NDIM == 3) Rc = Rc + (double)a.dU[(2 * NV + nv) * n + c];
       const double u0 = a.U0[nv * n + c];
       if (a.stage == 1) u[nv] = u0 + Rc;
       else u[nv] = a.w0 * u0 + a.w1 * a.Uc[nv * n + c] + a.wr * Rc;
     }
     if (a.stage == 1) {  // the CFL maximum is a stage-1 quantity
-      cdt = (double)a.Cdt[c] + (double)a.Cdt[n + c];
-      if (NDIM == 3) cdt = cdt + (double)a.Cdt[2 * n + c];
+      cdt = (double)a.Cdt[c];
+      if (!SUM) cdt = cdt + (double)a.Cdt[n + c];
+      if (!SUM && NDIM == 3) cdt = cdt + (double)a.Cdt[2 * n + c];
     }
     if constexpr (PHYS != PHYS_HD) {
       // 32-bit wrapped offsets of the index and its two successors along
@@ -2010,7 +2087,7 @@ template <int PHYS, int NV, int NDIM, typename CTT>
 __global__ void __launch_bounds__(256, finish_minb<CTT>()) finish_kernel(StageArgs<CTT> a, Grid3 g) {
   step_order();
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const double cdt = finish_cell<PHYS, NV, NDIM, CTT>(a, g, c);
+  const double cdt = finish_cell<PHYS, NV, NDIM, sum_directions<PHYS, CTT>(), CTT>(a, g, c);
   // per-warp maximum: a block-wide one (a barrier per block) made the FP64
   // finish 9% slower in stage 1 and 5% in stage 2 at 256^3
   if (a.stage == 1) warp_invdt_max(a.invdt_bits, cdt, threadIdx.x & 31);
