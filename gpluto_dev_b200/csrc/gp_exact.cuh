@@ -153,20 +153,22 @@ struct FloatArith {
   __device__ __forceinline__ void densities(float l, float r) { bad = l < 0.0f || r < 0.0f; }
 };
 
+static __device__ __noinline__ double quot_call(double a, double b) { return a / b; }
+
 // RN(a/b) for a divisor fixed over a launch, y = RN(1/b) formed once; the
 // operator where the dividend is not 0 or in [2^-700, 2^700].  The caller
 // vouches for b in [2^-200, 2^200] (y = 0 otherwise: the operator).
 __device__ __forceinline__ double fixed_quot(double a, double b, double y) {
   FastArith f;
-  const double p = f.quot(a, b, y);
-  return (f.bad || y == 0.0) ? a / b : p;
+  f.check(a);
+  const double p = f.quot_bpos(a, b, y);
+  return (f.bad || y == 0.0) ? quot_call(a, b) : p;
 }
 __device__ __forceinline__ float fixed_quot(float a, float b, float) { return a / b; }
 
 // 1/b for fixed_quot (host side), 0 when b is outside its range
 __host__ __device__ inline double fixed_inv(double b) {
-  const double m = b < 0 ? -b : b;
-  return (m >= 0x1p-200 && m <= 0x1p200) ? 1.0 / b : 0.0;
+  return (b >= 0x1p-200 && b <= 0x1p200) ? 1.0 / b : 0.0;
 }
 // 1/(gamma - 1) for the solvers, 0 (the operators) for a gamma out of
 // [1 + 2^-40, 2^40]: a pressure whose gamma p passed its test is then a

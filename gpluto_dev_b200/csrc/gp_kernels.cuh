@@ -296,14 +296,14 @@ constexpr int sweep_x_stage_doubles() {
              : XRow<NV>::SIZE * (SWEEP_THREADS / 32);
 }
 // y/z sweeps: a ring of four cells and two face fields per thread (PLM,
-// LimO3, WENO3), two cells and face fields otherwise
+// LimO3, WENO3), five cells (PPM), two cells and face fields otherwise
 // values SumStage keeps of a cell: flux differences (at most 6 with a field in
 // two directions) and the inverse-dt term
 template <int NV>
 constexpr int sum_slots() { return NV == 8 ? 7 : NV + 1; }
 template <int NV, int LIM = LIM_MC, bool SUM = false>
 constexpr int sweep_m_stage_doubles() {
-  return (((LIM == LIM_PPM || five_point<LIM>()) ? 2 * (NV + 1) : 4 * NV + 2) +
+  return ((LIM == LIM_PPM ? 5 * NV + 2 : five_point<LIM>() ? 2 * (NV + 1) : 4 * NV + 2) +
           (SUM ? 2 * sum_slots<NV>() : 0)) *
          SWEEP_THREADS;
 }
@@ -897,15 +897,17 @@ struct SumStage {
   }
 };
 
-// Piecewise parabolic y/z march: cells m-1, m, m+1 in registers, cell m+2
-// staged with cp.async (one iteration ahead: cell m+3 and face m+1 are
-// prefetched while face m is solved).  The constrained value of face m+1 is
-// formed from cells m-1..m+2 and carried to the next iteration as face m's.
+// Piecewise parabolic y/z march: a ring of five cells in shared memory (m-1
+// .. m+2 read while face m is solved, m+3 in flight), for the same reason as
+// in sweep_m_col.  The constrained value of face m+1 is formed from cells
+// m-1..m+2 and carried to the next iteration as face m's.
 template <int PHYS, int NV, int NDIM, int RS, int CT, int DIR, bool SUM, typename R,
           typename CTT>
 __device__ __forceinline__ void sweep_m_col_ppm(const StageArgs<CTT>& a, const Grid3& g, int i,
                                                 int t, int seg, int S, double* stg_, int tid) {
-  double(*stg)[NV + 1][SWEEP_THREADS] = reinterpret_cast<double(*)[NV + 1][SWEEP_THREADS]>(stg_);
+  double(*sv)[NV][SWEEP_THREADS] = reinterpret_cast<double(*)[NV][SWEEP_THREADS]>(stg_);
+  double(*sb)[SWEEP_THREADS] =
+      reinterpret_cast<double(*)[SWEEP_THREADS]>(stg_ + 5 * NV * SWEEP_THREADS);
   const int nd = (DIR == 1) ? g.ny : g.nz;
   const long long n = g.n;
   const R gamma = (R)a.gamma;
@@ -916,58 +918,96 @@ __device__ __forceinline__ void sweep_m_col_ppm(const StageArgs<CTT>& a, const G
                                       : i + (long long)g.nx * t;
     const int m0 = seg * S;
     const int m1 = min(m0 + S, nd);
-    auto stage = [&](int mcell, int mface, int b) {
-      const long long cc = base + (long long)gidx(mcell, nd, g.outflow, DIR) * stride;
+    auto stage_cell = [&](int m, int slot) {
+      const long long cc = base + (long long)gidx(m, nd, g.outflow, DIR) * stride;
 #pragma unroll
-      for (int nv = 0; nv < NV; nv++) cp_async8(&stg[b][nv][tid], a.V + nv * n + cc);
-      if constexpr (PHYS != PHYS_HD)
-        cp_async8(&stg[b][NV][tid], a.Bs[DIR] + base + (long long)gidx(mface, nd, g.outflow, DIR) * stride);
-      cp_async_commit();
+      for (int nv = 0; nv < NV; nv++) cp_async8(&sv[slot][nv][tid], a.V + nv * n + cc);
     };
-    SumStage<PHYS, NV, NDIM, SUM, CTT> ss{a, n, stg_ + 2 * (NV + 1) * SWEEP_THREADS, tid};
-    stage(m0 + 2, m0, 0);
-    R W0[NV], W1[NV], W2[NV], Fm[NV], vLn[NV], Fp[NV], cmp = R(0);
+    auto stage_face = [&](int m) {
+      if constexpr (PHYS != PHYS_HD)
+        cp_async8(&sb[m & 1][tid],
+                  a.Bs[DIR] + base + (long long)gidx(m, nd, g.outflow, DIR) * stride);
+    };
+    SumStage<PHYS, NV, NDIM, SUM, CTT> ss{a, n, stg_ + (5 * NV + 2) * SWEEP_THREADS, tid};
+    // slots q .. q+3 (mod 5) hold cells m-1 .. m+2
+    stage_cell(m0 - 1, 0);
+    stage_cell(m0, 1);
+    stage_cell(m0 + 1, 2);
+    cp_async_commit();
+    stage_cell(m0 + 2, 3);
+    stage_face(m0);
+    cp_async_commit();
+    // FP32 cells are converted once and stay in a window
+    constexpr bool kWindow = sizeof(R) == 4;
+    R Fm[NV], vLn[NV], Fp[NV], cmp = R(0), W0[NV], W1[NV], W2[NV];
     {
-      R q3[NV], q2[NV];
+      R q3[NV], q2[NV], w0[NV];
       load_cell<NV>(a.V, n, base + gidx(m0 - 3, nd, g.outflow, DIR) * stride, q3);
       load_cell<NV>(a.V, n, base + gidx(m0 - 2, nd, g.outflow, DIR) * stride, q2);
-      load_cell<NV>(a.V, n, base + gidx(m0 - 1, nd, g.outflow, DIR) * stride, W0);
-      load_cell<NV>(a.V, n, base + (long long)m0 * stride, W1);
-      load_cell<NV>(a.V, n, base + gidx(m0 + 1, nd, g.outflow, DIR) * stride, W2);
+      cp_async_wait1();
       R vrp[NV];
 #pragma unroll
       for (int nv = 0; nv < NV; nv++) {
-        const R fa = ppm_face(q3[nv], q2[nv], W0[nv], W1[nv]);   // face m0-1
-        Fm[nv] = ppm_face(q2[nv], W0[nv], W1[nv], W2[nv]);       // face m0
+        const R w1 = (R)sv[1][nv][tid], w2 = (R)sv[2][nv][tid];
+        w0[nv] = (R)sv[0][nv][tid];
+        const R fa = ppm_face(q3[nv], q2[nv], w0[nv], w1);   // face m0-1
+        Fm[nv] = ppm_face(q2[nv], w0[nv], w1, w2);           // face m0
         R dvp, dvm;
-        ppm_cell(W0[nv], fa, Fm[nv], dvp, dvm);                   // cell m0-1
-        vLn[nv] = W0[nv] + dvp;
-        vrp[nv] = W0[nv] + dvm;
+        ppm_cell(w0[nv], fa, Fm[nv], dvp, dvm);              // cell m0-1
+        vLn[nv] = w0[nv] + dvp;
+        vrp[nv] = w0[nv] + dvm;
         Fp[nv] = R(0);
+        if constexpr (kWindow) {
+          W0[nv] = w0[nv];
+          W1[nv] = w1;
+          W2[nv] = w2;
+        }
       }
-      if constexpr (PHYS == PHYS_RMHD) rmhd_vel_limit<NV>(W0, vrp, vLn);
+      if constexpr (PHYS == PHYS_RMHD) rmhd_vel_limit<NV>(w0, vrp, vLn);
     }
-    int buf = 0;
-    for (int m = m0; m <= m1; m++, buf ^= 1) {
-      if (m < m1) ss.load(base + (long long)m * stride, m & 1);
-      stage(m + 3, m + 1, buf ^ 1);   // prefetch for the next iteration
-      cp_async_wait1();
-      R vL[NV], vR[NV], F[NV], W3[NV];
-#pragma unroll
-      for (int nv = 0; nv < NV; nv++) {
-        W3[nv] = (R)stg[buf][nv][tid];                             // cell m+2
-        const R fn = ppm_face(W0[nv], W1[nv], W2[nv], W3[nv]);     // face m+1
-        R dvp, dvm;
-        ppm_cell(W1[nv], Fm[nv], fn, dvp, dvm);                   // cell m
-        vL[nv] = vLn[nv];
-        vR[nv] = W1[nv] + dvm;
-        vLn[nv] = W1[nv] + dvp;
-        Fm[nv] = fn;
+    int q = 0;
+    for (int m = m0; m <= m1; m++) {
+      const int q1 = q + 1 < 5 ? q + 1 : 0, q2 = q1 + 1 < 5 ? q1 + 1 : 0;
+      const int q3 = q2 + 1 < 5 ? q2 + 1 : 0, q4 = q3 + 1 < 5 ? q3 + 1 : 0;
+      if (m < m1) {   // prefetch for the next iteration
+        stage_cell(m + 3, q4);
+        stage_face(m + 1);
+        ss.load(base + (long long)m * stride, m & 1);
       }
-      if constexpr (PHYS == PHYS_RMHD) rmhd_vel_limit<NV>(W1, vR, vLn);
+      cp_async_commit();
+      cp_async_wait1();
+      R vL[NV], vR[NV], F[NV];
+      {
+        R w1[NV];
+#pragma unroll
+        for (int nv = 0; nv < NV; nv++) {
+          R w0, w2;                                                   // cells m-1, m+1
+          const R w3 = (R)sv[q3][nv][tid];                            // cell m+2
+          if constexpr (kWindow) {
+            w0 = W0[nv];
+            w1[nv] = W1[nv];
+            w2 = W2[nv];
+            W0[nv] = w1[nv];
+            W1[nv] = w2;
+            W2[nv] = w3;
+          } else {
+            w0 = (R)sv[q][nv][tid];
+            w1[nv] = (R)sv[q1][nv][tid];
+            w2 = (R)sv[q2][nv][tid];
+          }
+          const R fn = ppm_face(w0, w1[nv], w2, w3);                  // face m+1
+          R dvp, dvm;
+          ppm_cell(w1[nv], Fm[nv], fn, dvp, dvm);                     // cell m
+          vL[nv] = vLn[nv];
+          vR[nv] = w1[nv] + dvm;
+          vLn[nv] = w1[nv] + dvp;
+          Fm[nv] = fn;
+        }
+        if constexpr (PHYS == PHYS_RMHD) rmhd_vel_limit<NV>(w1, vR, vLn);
+      }
       R Bn = R(0);
       if constexpr (PHYS != PHYS_HD) {
-        Bn = (R)stg[buf][NV][tid];
+        Bn = (R)sb[m & 1][tid];
         vL[BX1 + DIR] = Bn;
         vR[BX1 + DIR] = Bn;
       }
@@ -987,13 +1027,9 @@ __device__ __forceinline__ void sweep_m_col_ppm(const StageArgs<CTT>& a, const G
                                     DIR, ss.get((m - 1) & 1, sum));
       }
 #pragma unroll
-      for (int nv = 0; nv < NV; nv++) {
-        W0[nv] = W1[nv];
-        W1[nv] = W2[nv];
-        W2[nv] = W3[nv];
-        Fp[nv] = F[nv];
-      }
+      for (int nv = 0; nv < NV; nv++) Fp[nv] = F[nv];
       cmp = cm;
+      q = q1;
     }
     cp_async_wait0();
   }

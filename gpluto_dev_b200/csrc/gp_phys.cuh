@@ -133,7 +133,7 @@ __device__ __forceinline__ R mp5_edge(R Fmm, R Fm, R F0, R Fp, R Fpp) {
   const R alpha = R(4), epsm = R(1.e-12);
   const R dFp = Fp - F0, dFm = F0 - Fm;
   R f = R(2) * Fmm - R(13) * Fm + R(47) * F0 + R(27) * Fp - R(3) * Fpp;  // Eq. (2.1)
-  f /= R(60);
+  f = fixed_quot(f, R(60), R(1.0 / 60.0));
   const R fMP = F0 + minmod(dFp, alpha * dFm);                          // Eq. (2.12)
   if ((f - F0) * (f - fMP) <= epsm) return f;
   const R d2m = Fmm + F0 - R(2) * Fm;
@@ -188,7 +188,7 @@ __device__ __forceinline__ R wenoz_edge(R Fmm, R Fm, R F0, R Fp, R Fpp) {
   const R f0 = R(2) * Fmm - R(7) * Fm + R(11) * F0;
   const R f1 = -Fm + R(5) * F0 + R(2) * Fp;
   const R f2 = R(2) * F0 + R(5) * Fp - Fpp;
-  return (w0 * f0 + w1 * f1 + w2 * f2) / R(6);
+  return fixed_quot(w0 * f0 + w1 * f1 + w2 * f2, R(6), R(1.0 / 6.0));
 }
 
 // 3-point edge values on a uniform grid of cell width dx, stencil ordered
@@ -260,7 +260,7 @@ __device__ __forceinline__ R edge5(R Fmm, R Fm, R F0, R Fp, R Fpp) {
 // of cell qp; both are this same expression, so it is computed once here.
 template <typename R>
 __device__ __forceinline__ R ppm_face(R qm, R q0, R qp, R qpp) {
-  R f = (-qm + R(7) * (q0 + qp) - qpp) / R(12);
+  R f = fixed_quot(-qm + R(7) * (q0 + qp) - qpp, R(12), R(1.0 / 12.0));
   return q0 + minmod(f - q0, qp - q0);
 }
 
@@ -284,8 +284,8 @@ __device__ __forceinline__ void ppm_cell(R v, R fm, R fp, R& dvp, R& dvm) {
 // to its right (dqp) and left (dqm) faces.
 template <typename R>
 __device__ __forceinline__ void par3_cell(R qm, R q0, R qp, R& dqp, R& dqm) {
-  R fp = (-qm + R(5) * q0 + R(2) * qp) / R(6);
-  R fm = (R(2) * qm + R(5) * q0 - qp) / R(6);
+  R fp = fixed_quot(-qm + R(5) * q0 + R(2) * qp, R(6), R(1.0 / 6.0));
+  R fm = fixed_quot(R(2) * qm + R(5) * q0 - qp, R(6), R(1.0 / 6.0));
   dqp = fp - q0;
   dqm = fm - q0;
   R dq = qp - q0;
