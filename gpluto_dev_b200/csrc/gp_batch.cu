@@ -219,6 +219,7 @@ struct gp_batch {
   std::map<size_t, size_t> free_list;  // offset -> size
   std::vector<BatchSlot> slots;        // host copy of the slot table
   std::vector<char> used;
+  std::vector<gp_tile_shape> shape;    // per slot as asked for (0: chosen from the whole batch)
   std::vector<size_t> off, bytes;
   BatchSlot* slots_d;
   BatchTile* tiles_d;
@@ -289,10 +290,9 @@ void free_batch(gp_batch* b) {
   if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
 }
 
-void apply_shape(BatchSlot& s, const gp_tile_shape* shape) {
-  const int seg = shape && shape->seg > 0 ? shape->seg : 32;
+void apply_shape(BatchSlot& s, int seg, int cpt) {
   s.seg = std::min(seg, std::max(s.ny, s.nz));
-  s.cpt = shape && shape->cells_per_thread > 0 ? std::min(shape->cells_per_thread, 64) : 2;
+  s.cpt = std::min(cpt, 64);
 }
 
 void tile_counts(BatchSlot& s) {
@@ -319,6 +319,25 @@ void tile_counts(BatchSlot& s) {
 // grid down, so that the EMF tiles of the largest (longest) grids complete
 // first.
 int rebuild_tiles(gp_batch* b) {
+  // Shapes of the slots that ask for none: the longest march (<= 32 cells) and
+  // the most cells a thread (<= 16) that still give the launches' resident
+  // blocks about a tile each, since a tile's own overhead is a few
+  // microseconds.  128 grids of 64 to 512 cells a side: 16 cells a thread 2893
+  // us a step, 2 cells 3361; 24 grids of 64 to 256: march 8 and 4 cells a
+  // thread 311 us, 32 and 2 431.
+  long long cells = 0;
+  for (int i = 0; i < b->max_slots; i++)
+    if (b->used[i]) cells += b->slots[i].n;
+  int seg = 32, cpt = 16;
+  while (seg > 4 && cells < (long long)seg * gp::BATCH_THREADS * b->ctas_full) seg /= 2;
+  while (cpt > 1 && cells * 10 < 7LL * cpt * gp::BATCH_THREADS * b->cell_ctas) cpt /= 2;
+  for (int i = 0; i < b->max_slots; i++) {
+    if (!b->used[i]) continue;
+    const gp_tile_shape& t = b->shape[i];
+    apply_shape(b->slots[i], t.seg > 0 ? t.seg : seg,
+                t.cells_per_thread > 0 ? t.cells_per_thread : cpt);
+    tile_counts(b->slots[i]);
+  }
   std::vector<int> order;
   for (int i = 0; i < b->max_slots; i++)
     if (b->used[i]) order.push_back(i);
@@ -417,6 +436,7 @@ int gp_batch_create(size_t pool_bytes, int max_slots, int ctas, void* stream, gp
   b->bias_need = 0;
   b->slots.assign(max_slots, BatchSlot{});
   b->used.assign(max_slots, 0);
+  b->shape.assign(max_slots, gp_tile_shape{0, 0});
   b->off.assign(max_slots, 0);
   b->bytes.assign(max_slots, 0);
   b->stream = static_cast<cudaStream_t>(stream);
@@ -540,7 +560,6 @@ int gp_batch_add(gp_batch* b, const gp_grid_desc* grid, const gp_scheme* scheme,
   s.ny = grid->nint[1];
   s.nz = grid->ndim == 3 ? grid->nint[2] : 1;
   s.n = n;
-  apply_shape(s, shape);
   s.cfl = scheme->cfl;
   s.cfl_max_var = scheme->cfl_max_var;
   for (int d = 0; d < 3; d++) {
@@ -549,7 +568,6 @@ int gp_batch_add(gp_batch* b, const gp_grid_desc* grid, const gp_scheme* scheme,
     if (!(s.dx[d] > 0.0)) s.dx[d] = 1.0;
   }
   s.sc = sc;
-  tile_counts(s);
   for (int bc = 0; bc < 3; bc++) {
     const int b0 = bc, b1 = (bc + 1) % 3, b2 = (bc + 2) % 3;
     for (int stage = 1; stage <= 2; stage++) {
@@ -612,6 +630,7 @@ int gp_batch_add(gp_batch* b, const gp_grid_desc* grid, const gp_scheme* scheme,
   }
   b->slots[idx] = s;
   b->used[idx] = 1;
+  b->shape[idx] = shape ? *shape : gp_tile_shape{0, 0};
   b->off[idx] = off;
   b->bytes[idx] = L.bytes;
   b->sc_h[idx] = hs;
@@ -623,9 +642,7 @@ int gp_batch_add(gp_batch* b, const gp_grid_desc* grid, const gp_scheme* scheme,
 int gp_batch_set_shape(gp_batch* b, int slot, const gp_tile_shape* shape) {
   if (!b || slot < 0 || slot >= b->max_slots || !b->used[slot])
     return gp::fail(GP_ERR_INVALID, "no such slot");
-  BatchSlot& s = b->slots[slot];
-  apply_shape(s, shape);
-  tile_counts(s);
+  b->shape[slot] = shape ? *shape : gp_tile_shape{0, 0};
   b->dirty = true;
   return GP_OK;
 }

@@ -272,7 +272,7 @@ int gp_advance_step_noalloc(const gp_grid_desc *grid, const gp_scheme *scheme,
    --------------------------------------------------------------------- */
 typedef struct gp_batch gp_batch;
 
-/* Tile shape of one slot (0 = default): `seg` is the pencil segment of the
+/* Tile shape of one slot (0 = chosen from all the batch holds): `seg` is the pencil segment of the
    y/z sweeps (cells one thread marches), `cells_per_thread` the cells each
    thread of an edge-EMF or finish tile handles. */
 typedef struct gp_tile_shape {
