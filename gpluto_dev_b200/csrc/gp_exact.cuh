@@ -127,30 +127,12 @@ struct FastArith {
     const double g = __dmul_rn(a, y1);
     return __fma_rn(__fma_rn(-g, g, a), __dmul_rn(0.5, y1), g);
   }
-  // star densities: root() marks the negative ones
-  __device__ __forceinline__ void densities(double, double) {}
   // root of a >= +0
   __device__ __forceinline__ double root0(double a) {
     const bool zero = __double_as_longlong(a) == 0;
     const double r = root(zero ? 1.0 : a);
     return zero ? a : r;
   }
-};
-
-// FP32 of the mixed form: one approximate reciprocal per divisor (the units
-// compile with approximate division, so a quotient is such a product there
-// too).  `bad` only marks negative star densities (the HLL fallback).
-struct FloatArith {
-  static constexpr bool FAST = true;
-  bool bad = false;
-  __device__ __forceinline__ float inv_pos(float b) { return 1.0f / b; }
-  __device__ __forceinline__ float inv_in(float b) { return 1.0f / b; }
-  __device__ __forceinline__ void check(float) {}
-  __device__ __forceinline__ float quot_pos(float a, float, float y) { return a * y; }
-  __device__ __forceinline__ float quot_bpos(float a, float, float y) { return a * y; }
-  __device__ __forceinline__ float div_any(float a, float b) { return a / b; }
-  __device__ __forceinline__ float root(float a) { return sqrtf(a); }
-  __device__ __forceinline__ void densities(float l, float r) { bad = l < 0.0f || r < 0.0f; }
 };
 
 static __device__ __noinline__ double quot_call(double a, double b) { return a / b; }

@@ -113,14 +113,32 @@ __device__ __forceinline__ void cp_async_wait0() {
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
-// Programmatic dependent launch: a kernel of the step lets the next one's
-// blocks be placed as soon as all of its own are running, and touches memory
-// only after every kernel before it has completed.  Small grids are bound by
-// the launches' latency (2-D MHD 64^2: step 82 -> 72 us; 256^2, ten steps: 808
-// -> 704 us).
-__device__ __forceinline__ void step_order() {
+// Programmatic dependent launch.  launch_next lets the next kernel's blocks be
+// placed once all blocks of this one have called it; wait_before returns when
+// every kernel launched before this one has completed and its writes are
+// visible.  A kernel calls launch_next and wait_before first of all.  With
+// OVERLAP the sweeps of a stage, which do not read one another's results, run
+// side by side:
+//   * the x-sweep calls wait_before first, so that the kernel it lets in
+//     starts after the state it needs is complete;
+//   * the y and z sweeps start at once and call wait_before last, so that
+//     their own completion means the sweep's before them.  (A kernel of its
+//     own: the call at the end cost the large grids' one 64 bytes of spills
+//     and 3%.)
+// Small grids are bound by the launches' latency and by each sweep's own chain
+// (2-D MHD 64^2: step 82 -> 72 us with the launches, 63 with the sweeps
+// overlapped; 256^2, ten steps: 808 -> 706 -> 684; 61x47x53, five steps: 941 ->
+// 905 -> 831).  The host does both up to 2^20 cells (kEarlyCells) and does not
+// overlap RMHD: RMHD 90x72x60 lost 12% (two long codes in one instruction cache).
+__device__ __forceinline__ void launch_next() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_before() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void step_order() {
+  launch_next();
+  wait_before();
 }
 
 #ifndef GP_SWEEP_MINB
@@ -130,11 +148,11 @@ constexpr int SWEEP_THREADS = 128;
 
 // Resident 128-thread blocks per SM the sweep kernels are compiled for
 // (register budget 65536 / (128 * blocks)), measured at 256^3 on 3-D MHD:
-// FP64 x-sweep 3 (168 registers), FP64 y/z sweeps 4 (128), mixed form 5
-// (102).  The relativistic solver (FP64 in both forms) runs its x-sweep at
-// 2 (5.01 -> 4.83 ms FP64, 4.33 -> 4.06 ms mixed at 192^3: fewer warps
-// walking its long code at once) and its y/z sweeps at 3 (at 2 they lost
-// 4%).
+// FP64 x-sweep 3 (168 registers; at 4 1084 -> 1142 us), FP64 y/z sweeps 4 (128;
+// at 3 the same), mixed form 5 (102; at 6 x 568 -> 779 us).  The relativistic
+// solver's long code runs at 2, fewer warps walking it at once (192^3 FP64 y/z
+// 3617/4335 us at 3, 3152/3885 at 2); its mixed y/z sweeps stay at 3, which
+// fits small grids' waves better (90x72x60: 260 against 314 us).
 template <int PHYS, typename R>
 constexpr int sweep_x_minb() {
   return PHYS == PHYS_RMHD ? 2 : (sizeof(R) == 4 ? 5 : 3);
@@ -167,8 +185,9 @@ __device__ __forceinline__ R riemann(const R* vl, const R* vr, R* flux, R gamma,
                                      CTFace<R>& ct, uint32_t& err) {
   if constexpr (PHYS == PHYS_MHD) {
     R cm;
-    if constexpr (RS == RS_HLLD)
-      cm = mhd_hlld_face<DIR, CT>(vl, vr, flux, gamma, ygm, Bn, ct);
+    if constexpr (RS == RS_HLLD && sizeof(R) == sizeof(double))
+      cm = mhd_hlld_fp64<DIR, CT>(vl, vr, flux, gamma, ygm, Bn, ct);
+    else if constexpr (RS == RS_HLLD) cm = mhd_hlld<DIR, CT>(vl, vr, flux, gamma, Bn, ct);
     else if constexpr (RS == RS_TVDLF) cm = mhd_tvdlf<DIR>(vl, vr, flux, gamma, ct);
     else if constexpr (RS == RS_HLLC) cm = mhd_hllc<DIR>(vl, vr, flux, gamma, ct);
     else cm = mhd_hll<DIR>(vl, vr, flux, gamma, ct);
@@ -293,7 +312,7 @@ template <int NV, int LIM = LIM_MC>
 constexpr int sweep_x_stage_doubles() {
   return (LIM == LIM_PPM || five_point<LIM>())
              ? 2 * (2 * NV + 1) * SWEEP_THREADS + 2 * (SWEEP_THREADS / 32) * NV
-             : XRow<NV>::SIZE * (SWEEP_THREADS / 32);
+             : XRow<NV>::SIZE * (SWEEP_THREADS / 32);  // FP32: 2 * (2 * NV + 1) * 128 of them
 }
 // y/z sweeps: a ring of four cells and two face fields per thread (PLM,
 // LimO3, WENO3), five cells (PPM), two cells and face fields otherwise
@@ -669,6 +688,180 @@ __device__ __forceinline__ void cell_edges(const R* vm, const R* v0, const R* vp
   }
 }
 
+// The FP32 forms of the x-row and the y/z march (PLM and the 3-point
+// reconstructions): neighbours by shuffle with a carry in every lane, cells in a
+// register window.  At half the registers they do not spill, and each cell is
+// converted from FP64 once.
+template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, typename R, typename CTT>
+__device__ __forceinline__ void sweep_x_row_f32(const StageArgs<CTT>& a, const Grid3& g, int row,
+                                                double* stg_, int tid) {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int SL = 2 * NV + 1;  // staged doubles per lane: V[f], V[f+1], Bs[f]
+  double(*stg)[SL][SWEEP_THREADS] = reinterpret_cast<double(*)[SL][SWEEP_THREADS]>(stg_);
+  const int lane = tid & 31;
+  if (row >= g.ny * g.nz) return;  // warp-uniform
+  const int nx = g.nx;
+  const unsigned ob = g.outflow;
+  // faces solved: nx (periodic: face nx is face 0) or nx+1 (outflow high side)
+  const int nf = nx + (int)((ob >> 1) & 1u);
+  const long long n = g.n;
+  const long long rb = (long long)row * nx;
+  const R gamma = (R)a.gamma;
+
+  // carried state of cell c0-1 (uniform over lanes)
+  R pV[NV], pVLn[NV], pF[NV], pCm = R(0);
+  {
+    R vm[NV], v0[NV], vp[NV];
+    load_cell<NV>(a.V, n, rb + gidx(-2, nx, ob, 0), vm);
+    load_cell<NV>(a.V, n, rb + gidx(-1, nx, ob, 0), v0);
+    load_cell<NV>(a.V, n, rb + 0, vp);
+    R pVR[NV];
+    if constexpr (three_point<LIM>()) {
+      const R dx = (R)a.dx[0];
+#pragma unroll
+      for (int nv = 0; nv < NV; nv++) {
+        pV[nv] = v0[nv];
+        pVLn[nv] = edge3<LIM>(vm[nv], v0[nv], vp[nv], dx);
+        pVR[nv] = edge3<LIM>(vp[nv], v0[nv], vm[nv], dx);
+        pF[nv] = R(0);
+      }
+      const R qm[2] = {vm[RHO], vm[NV - 1]}, qp[2] = {vp[RHO], vp[NV - 1]};
+      mp5_fallback<PHYS, NV>(v0, qm, qp, pVR, pVLn);
+    } else {
+#pragma unroll
+      for (int nv = 0; nv < NV; nv++) {
+        R dv = limit<LIM>(vp[nv] - v0[nv], v0[nv] - vm[nv]);
+        pV[nv] = v0[nv];
+        pVLn[nv] = v0[nv] + R(0.5) * dv;
+        pVR[nv] = v0[nv] - R(0.5) * dv;
+        pF[nv] = R(0);
+      }
+      if constexpr (PHYS == PHYS_RMHD) rmhd_vel_limit<NV>(v0, pVR, pVLn);
+    }
+  }
+  R fF[NV], fCm = R(0);  // flux of face 0 (lane 0 of the first chunk)
+  R F[NV], cm = R(0);
+#pragma unroll
+  for (int nv = 0; nv < NV; nv++) { fF[nv] = R(0); F[nv] = R(0); }
+  uint32_t err = 0;
+
+  // stage chunk c0 into buffer b: V[f], V[f+1] (lanes that cannot take it
+  // from the next lane), Bs[f]
+  auto stage_chunk = [&](int c0, int b) {
+    const int f = c0 + lane;
+    const int fc = f < nx ? f : nx - 1;
+#pragma unroll
+    for (int nv = 0; nv < NV; nv++) cp_async8(&stg[b][nv][tid], a.V + nv * n + rb + fc);
+    if (lane == 31 || f + 1 >= nf) {
+      const int fp = gidx(fc + 1, nx, ob, 0);
+#pragma unroll
+      for (int nv = 0; nv < NV; nv++) cp_async8(&stg[b][NV + nv][tid], a.V + nv * n + rb + fp);
+    }
+    if constexpr (PHYS != PHYS_HD) cp_async8(&stg[b][2 * NV][tid], a.Bs[0] + rb + fc);
+    cp_async_commit();
+  };
+  stage_chunk(0, 0);
+  int buf = 0;
+  for (int c0 = 0; c0 < nf; c0 += 32, buf ^= 1) {
+    const int f = c0 + lane;
+    const bool act = f < nf;
+    stage_chunk(c0 + 32 < nf ? c0 + 32 : c0, buf ^ 1);   // prefetch the next chunk
+    cp_async_wait1();
+    R Vc[NV], Vm1[NV], Vp1[NV], vL[NV], vR[NV], vLn[NV];
+    const bool selfp1 = (lane == 31) || (f + 1 >= nf);
+#pragma unroll
+    for (int nv = 0; nv < NV; nv++) {
+      Vc[nv] = (R)stg[buf][nv][tid];
+      if (selfp1) Vp1[nv] = (R)stg[buf][NV + nv][tid];
+    }
+    if constexpr (three_point<LIM>()) {
+      const R dx = (R)a.dx[0];
+#pragma unroll
+      for (int nv = 0; nv < NV; nv++) {
+        R up = __shfl_up_sync(FULL, Vc[nv], 1);
+        R dn = __shfl_down_sync(FULL, Vc[nv], 1);
+        Vm1[nv] = (lane == 0) ? pV[nv] : up;
+        if (!selfp1) Vp1[nv] = dn;
+        vR[nv] = edge3<LIM>(Vp1[nv], Vc[nv], Vm1[nv], dx);
+        vLn[nv] = edge3<LIM>(Vm1[nv], Vc[nv], Vp1[nv], dx);
+      }
+      const R qm[2] = {Vm1[RHO], Vm1[NV - 1]}, qp[2] = {Vp1[RHO], Vp1[NV - 1]};
+      mp5_fallback<PHYS, NV>(Vc, qm, qp, vR, vLn);
+    } else {
+#pragma unroll
+      for (int nv = 0; nv < NV; nv++) {
+        R up = __shfl_up_sync(FULL, Vc[nv], 1);
+        R dn = __shfl_down_sync(FULL, Vc[nv], 1);
+        Vm1[nv] = (lane == 0) ? pV[nv] : up;
+        if (!selfp1) Vp1[nv] = dn;
+        R dv = limit<LIM>(Vp1[nv] - Vc[nv], Vc[nv] - Vm1[nv]);
+        vR[nv] = Vc[nv] - R(0.5) * dv;
+        vLn[nv] = Vc[nv] + R(0.5) * dv;
+      }
+      if constexpr (PHYS == PHYS_RMHD) rmhd_vel_limit<NV>(Vc, vR, vLn);
+    }
+#pragma unroll
+    for (int nv = 0; nv < NV; nv++) {
+      R l = __shfl_up_sync(FULL, vLn[nv], 1);
+      vL[nv] = (lane == 0) ? pVLn[nv] : l;
+    }
+    R Bn = R(0);
+    if constexpr (PHYS != PHYS_HD) {
+      Bn = (R)stg[buf][2 * NV][tid];  // Src/States/plm_states.cpp:184-189
+      vL[BX1] = Bn;
+      vR[BX1] = Bn;
+    }
+    CTFace<R> ct;
+    uint32_t fe = 0;
+    cm = riemann<PHYS, RS, CT, 0>(vL, vR, F, gamma, (R)a.inv_gm1, Bn, ct, fe);
+#pragma unroll
+    for (int nv = 0; nv < NV; nv++)
+      if (act && rhs_var<PHYS, NDIM>(nv) && isnan(F[nv])) fe |= ERR_NAN | ERR_QUIT;
+    if (fe && face_counts(g, 0, f, 1, row % g.ny, 2, row / g.ny)) err |= fe;
+    if constexpr (PHYS != PHYS_HD) {
+      if (act) store_ct<CT>(a, 0, rb + f, ct);
+    }
+    // flux of face f-1 and cell update of cell f-1
+    R Fm1[NV];
+#pragma unroll
+    for (int nv = 0; nv < NV; nv++) {
+      R t = __shfl_up_sync(FULL, F[nv], 1);
+      Fm1[nv] = (lane == 0) ? pF[nv] : t;
+    }
+    R cmm1;
+    {
+      R t = __shfl_up_sync(FULL, cm, 1);
+      cmm1 = (lane == 0) ? pCm : t;
+    }
+    if (act && f >= 1)
+      cell_update<PHYS, NV, NDIM>(a, n, rb + (f - 1), Fm1, F, cmm1, cm, 0);
+    if (c0 == 0) {
+#pragma unroll
+      for (int nv = 0; nv < NV; nv++) fF[nv] = F[nv];
+      fCm = cm;
+    }
+#pragma unroll
+    for (int nv = 0; nv < NV; nv++) {
+      pV[nv] = __shfl_sync(FULL, Vc[nv], 31);
+      pVLn[nv] = __shfl_sync(FULL, vLn[nv], 31);
+      pF[nv] = __shfl_sync(FULL, F[nv], 31);
+    }
+    pCm = __shfl_sync(FULL, cm, 31);
+  }
+  cp_async_wait0();
+  // periodic: cell nx-1 uses F[nx-1] (lane (nx-1)%32 of the last chunk) and
+  // F[nx] = F[0]; with an outflow high side face nx was solved in the loop
+  if (nf == nx) {
+    R F0[NV];
+#pragma unroll
+    for (int nv = 0; nv < NV; nv++) F0[nv] = __shfl_sync(FULL, fF[nv], 0);
+    R cm0 = __shfl_sync(FULL, fCm, 0);
+    if (lane == ((nx - 1) & 31))
+      cell_update<PHYS, NV, NDIM>(a, n, rb + (nx - 1), F, F0, cm, cm0, 0);
+  }
+  if (err) atomicOr(a.err, err);
+}
+
 // The cells [s0, s1) of one x-row by one warp.  Chunks of 32 faces: lane l
 // solves face f = c0 + l and updates cell f-1.  Cells (with a halo of one on
 // each side), right edge values and fluxes pass between the lanes and from
@@ -842,12 +1035,18 @@ __device__ __forceinline__ void sweep_x_row(const StageArgs<CTT>& a, const Grid3
   if (err) atomicOr(a.err, err);
 }
 
-template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, typename R, typename CTT>
+// WHOLE: one row a warp, FP32 (the host's x_segments gave one part)
+template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, bool WHOLE, typename R, typename CTT>
 __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_x_minb<PHYS, R>()))
     sweep_x_kernel(StageArgs<CTT> a, Grid3 g, int nseg) {
   __shared__ double stg[sweep_x_stage_doubles<NV, LIM>()];
-  step_order();
+  wait_before();
+  launch_next();
   const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if constexpr (WHOLE && LIM != LIM_PPM && !five_point<LIM>()) {
+    sweep_x_row_f32<PHYS, NV, NDIM, RS, CT, LIM, R, CTT>(a, g, w, stg, threadIdx.x);
+    return;
+  }
   const int row = w / nseg, q = w - row * nseg;
   sweep_x_row<PHYS, NV, NDIM, RS, CT, LIM, R, CTT>(a, g, row, (int)((long long)g.nx * q / nseg),
                                                    (int)((long long)g.nx * (q + 1) / nseg), stg,
@@ -1133,6 +1332,117 @@ __device__ __forceinline__ void sweep_m_col_mp5(const StageArgs<CTT>& a, const G
   if (err) atomicOr(a.err, err);
 }
 
+template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, typename R,
+          typename CTT>
+__device__ __forceinline__ void sweep_m_col_f32(const StageArgs<CTT>& a, const Grid3& g, int i, int t,
+                                            int seg, int S, double* stg_, int tid) {
+  double(*stg)[NV + 1][SWEEP_THREADS] = reinterpret_cast<double(*)[NV + 1][SWEEP_THREADS]>(stg_);
+  const int nd = (DIR == 1) ? g.ny : g.nz;
+  const long long n = g.n;
+  const R gamma = (R)a.gamma;
+  uint32_t err = 0;
+  if (i < g.nx) {
+    const long long stride = (DIR == 1) ? (long long)g.nx : (long long)g.nx * g.ny;
+    const long long base = (DIR == 1) ? i + (long long)g.nx * g.ny * t
+                                      : i + (long long)g.nx * t;
+    const int m0 = seg * S;
+    const int m1 = min(m0 + S, nd);
+    auto stage = [&](int mcell, int mface, int b) {
+      const long long cc = base + (long long)gidx(mcell, nd, g.outflow, DIR) * stride;
+#pragma unroll
+      for (int nv = 0; nv < NV; nv++) cp_async8(&stg[b][nv][tid], a.V + nv * n + cc);
+      if constexpr (PHYS != PHYS_HD)
+        cp_async8(&stg[b][NV][tid], a.Bs[DIR] + base + (long long)gidx(mface, nd, g.outflow, DIR) * stride);
+      cp_async_commit();
+    };
+    stage(m0 + 1, m0, 0);
+    R Vp[NV], Vc[NV], vLn[NV], Fp[NV], cmp = R(0);
+    {
+      R vmm[NV];
+      load_cell<NV>(a.V, n, base + gidx(m0 - 2, nd, g.outflow, DIR) * stride, vmm);
+      load_cell<NV>(a.V, n, base + gidx(m0 - 1, nd, g.outflow, DIR) * stride, Vp);
+      load_cell<NV>(a.V, n, base + (long long)m0 * stride, Vc);
+      R vrp[NV];
+      if constexpr (three_point<LIM>()) {
+        const R dx = (R)a.dx[DIR];
+#pragma unroll
+        for (int nv = 0; nv < NV; nv++) {
+          vLn[nv] = edge3<LIM>(vmm[nv], Vp[nv], Vc[nv], dx);
+          vrp[nv] = edge3<LIM>(Vc[nv], Vp[nv], vmm[nv], dx);
+          Fp[nv] = R(0);
+        }
+        const R qm[2] = {vmm[RHO], vmm[NV - 1]}, qp[2] = {Vc[RHO], Vc[NV - 1]};
+        mp5_fallback<PHYS, NV>(Vp, qm, qp, vrp, vLn);
+      } else {
+#pragma unroll
+        for (int nv = 0; nv < NV; nv++) {
+          R dv = limit<LIM>(Vc[nv] - Vp[nv], Vp[nv] - vmm[nv]);
+          vLn[nv] = Vp[nv] + R(0.5) * dv;
+          vrp[nv] = Vp[nv] - R(0.5) * dv;
+          Fp[nv] = R(0);
+        }
+        if constexpr (PHYS == PHYS_RMHD) rmhd_vel_limit<NV>(Vp, vrp, vLn);
+      }
+    }
+    int buf = 0;
+    for (int m = m0; m <= m1; m++, buf ^= 1) {
+      stage(min(m + 2, m1 + 1), min(m + 1, m1), buf ^ 1);   // prefetch for the next iteration
+      cp_async_wait1();
+      R Vn[NV], vL[NV], vR[NV], F[NV];
+      if constexpr (three_point<LIM>()) {
+        const R dx = (R)a.dx[DIR];
+#pragma unroll
+        for (int nv = 0; nv < NV; nv++) {
+          Vn[nv] = (R)stg[buf][nv][tid];
+          vL[nv] = vLn[nv];
+          vR[nv] = edge3<LIM>(Vn[nv], Vc[nv], Vp[nv], dx);
+          vLn[nv] = edge3<LIM>(Vp[nv], Vc[nv], Vn[nv], dx);
+        }
+        const R qm[2] = {Vp[RHO], Vp[NV - 1]}, qp[2] = {Vn[RHO], Vn[NV - 1]};
+        mp5_fallback<PHYS, NV>(Vc, qm, qp, vR, vLn);
+      } else {
+#pragma unroll
+        for (int nv = 0; nv < NV; nv++) {
+          Vn[nv] = (R)stg[buf][nv][tid];
+          R dv = limit<LIM>(Vn[nv] - Vc[nv], Vc[nv] - Vp[nv]);
+          vL[nv] = vLn[nv];
+          vR[nv] = Vc[nv] - R(0.5) * dv;
+          vLn[nv] = Vc[nv] + R(0.5) * dv;
+        }
+        if constexpr (PHYS == PHYS_RMHD) rmhd_vel_limit<NV>(Vc, vR, vLn);
+      }
+      R Bn = R(0);
+      if constexpr (PHYS != PHYS_HD) {
+        Bn = (R)stg[buf][NV][tid];
+        vL[BX1 + DIR] = Bn;
+        vR[BX1 + DIR] = Bn;
+      }
+      CTFace<R> ct;
+      uint32_t fe = 0;
+      R cm = riemann<PHYS, RS, CT, DIR>(vL, vR, F, gamma, (R)a.inv_gm1, Bn, ct, fe);
+#pragma unroll
+      for (int nv = 0; nv < NV; nv++)
+        if (rhs_var<PHYS, NDIM>(nv) && isnan(F[nv])) fe |= ERR_NAN | ERR_QUIT;
+      if (fe && face_counts(g, DIR, m, 0, i, DIR == 1 ? 2 : 1, t)) err |= fe;
+      if constexpr (PHYS != PHYS_HD) {
+        if (m < m1) store_ct<CT>(a, DIR, base + (long long)gidx(m, nd, g.outflow, DIR) * stride, ct);
+      }
+      if (m > m0)
+        cell_update<PHYS, NV, NDIM>(a, n, base + (long long)(m - 1) * stride, Fp, F, cmp, cm,
+                                    DIR);
+#pragma unroll
+      for (int nv = 0; nv < NV; nv++) {
+        Vp[nv] = Vc[nv];
+        Vc[nv] = Vn[nv];
+        Fp[nv] = F[nv];
+      }
+      cmp = cm;
+    }
+    cp_async_wait0();
+  }
+  if (err) atomicOr(a.err, err);
+}
+
 // One (x column i, transverse index t, pencil segment seg) per thread: t is
 // k for DIR=1 and j for DIR=2; the segment covers cells [seg*S, seg*S+S).
 // `stg_` is the block's staging area (sweep_m_stage_doubles<NV>() doubles).
@@ -1149,6 +1459,10 @@ __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3
                                                                       tid);
     return;
   }
+  if constexpr (sizeof(R) == 4) {
+    sweep_m_col_f32<PHYS, NV, NDIM, RS, CT, LIM, DIR, R, CTT>(a, g, i, t, seg, S, stg_, tid);
+    return;
+  }
   // Ring of four cells (cell m in slot m & 3) and of two face fields: a
   // cell's three readers take it from shared memory, so that no cell is live
   // in registers across the Riemann solver (FP64 256^3, with the straight-line
@@ -1162,8 +1476,7 @@ __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3
   const R gamma = (R)a.gamma;
   uint32_t err = 0;
   if (i < g.nx) {
-    // 32-bit cell indexes (grids hold fewer than 2^31 cells): FP32 y/z 424/432
-    // -> 413/415 us at 256^3 against 64-bit ones, FP64 the same
+    // 32-bit cell indexes (grids hold fewer than 2^31 cells)
     const unsigned stride = (DIR == 1) ? (unsigned)g.nx : (unsigned)g.nx * g.ny;
     const unsigned base = (DIR == 1) ? i + (unsigned)g.nx * g.ny * t : i + (unsigned)g.nx * t;
     const int m0 = seg * S;
@@ -1189,22 +1502,13 @@ __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3
     stage_cell(m0 + 1);
     stage_face(m0);
     cp_async_commit();
-    // FP32 cells (half the registers) are converted once and stay in a window
-    constexpr bool kWindow = sizeof(R) == 4;
-    R vLn[NV], Fp[NV], cmp = R(0), W0[NV], W1[NV];
+    R vLn[NV], Fp[NV], cmp = R(0);
     {
       R vm[NV], v0[NV], vp[NV], w[NV];
       load_cell<NV>(a.V, n, base + gidx(m0 - 2, nd, g.outflow, DIR) * stride, vm);
       cp_async_wait1();
       cell(m0 - 1, v0);
       cell(m0, vp);
-      if constexpr (kWindow) {
-#pragma unroll
-        for (int nv = 0; nv < NV; nv++) {
-          W0[nv] = v0[nv];
-          W1[nv] = vp[nv];
-        }
-      }
       cell_edges<PHYS, NV, LIM>(vm, v0, vp, (R)a.dx[DIR], w, vLn);
 #pragma unroll
       for (int nv = 0; nv < NV; nv++) Fp[nv] = R(0);
@@ -1220,19 +1524,9 @@ __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3
       R vL[NV], vR[NV], F[NV];
       {
         R vm[NV], v0[NV], vp[NV];
+        cell(m - 1, vm);
+        cell(m, v0);
         cell(m + 1, vp);
-        if constexpr (kWindow) {
-#pragma unroll
-          for (int nv = 0; nv < NV; nv++) {
-            vm[nv] = W0[nv];
-            v0[nv] = W1[nv];
-            W0[nv] = v0[nv];
-            W1[nv] = vp[nv];
-          }
-        } else {
-          cell(m - 1, vm);
-          cell(m, v0);
-        }
 #pragma unroll
         for (int nv = 0; nv < NV; nv++) vL[nv] = vLn[nv];
         cell_edges<PHYS, NV, LIM>(vm, v0, vp, (R)a.dx[DIR], vR, vLn);
@@ -1273,12 +1567,14 @@ __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3
 // segments innermost, with the (x, t) columns numbered together (col = cb *
 // SWEEP_THREADS + thread, i = col % nx, t = col / nx), so that no block is
 // part-empty.
-template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, typename R, typename CTT>
+template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, bool OVERLAP, typename R,
+          typename CTT>
 __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_m_minb<PHYS, R>()))
     sweep_m_kernel(StageArgs<CTT> a, Grid3 g, int S, bool flat) {
   constexpr bool SUM = sum_directions<PHYS, CTT>();
   __shared__ double stg[sweep_m_stage_doubles<NV, LIM, SUM>()];
-  step_order();
+  launch_next();
+  if (!OVERLAP) wait_before();
   const int nd = (DIR == 1) ? g.ny : g.nz;
   const int nseg = (nd + S - 1) / S;
   int i, t, seg;
@@ -1297,6 +1593,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_m_minb<PHYS, R>()))
   }
   sweep_m_col<PHYS, NV, NDIM, RS, CT, LIM, DIR, SUM, R, CTT>(a, g, i, t, seg, S, stg,
                                                              threadIdx.x);
+  if (OVERLAP) wait_before();
 }
 
 // ---------------------------------------------------------------------

@@ -68,9 +68,15 @@ static StageArgs<CTT> make_args(const StageDesc& d) {
   return a;
 }
 
-// Launch in stream order, the next launch's blocks placed early (step_order)
+// Grids up to this many cells are launched early and overlap their sweeps: at
+// 256^3 early launches cost the mixed step 1.5% and the FP64 step 1%.
+constexpr long long kEarlyCells = 1LL << 20;
+
+// Launch in stream order, on a grid of at most kEarlyCells cells with its blocks
+// placed while the kernel before drains (step_order)
 template <typename... K, typename... A>
-static void launch(void (*k)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+static void launch(long long cells, void (*k)(K...), dim3 grid, dim3 block, size_t smem,
+                   cudaStream_t s, A... args) {
   cudaLaunchAttribute early;
   early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   early.val.programmaticStreamSerializationAllowed = 1;
@@ -80,7 +86,7 @@ static void launch(void (*k)(K...), dim3 grid, dim3 block, size_t smem, cudaStre
   c.dynamicSmemBytes = smem;
   c.stream = s;
   c.attrs = &early;
-  c.numAttrs = 1;
+  c.numAttrs = cells <= kEarlyCells ? 1 : 0;
   cudaLaunchKernelEx(&c, k, K(args)...);
 }
 
@@ -142,7 +148,18 @@ static void launch_m(const StageArgs<CTT>& a, const Grid3& g, int nt, int nd, cu
   pre();
   const bool flat = g.nx % SWEEP_THREADS != 0 || (long long)nt * nseg > 65535;
   const dim3 grid = flat ? dim3((unsigned)(cols * nseg)) : dim3(g.nx / SWEEP_THREADS, nt * nseg);
-  launch(sweep_m_kernel<PHYS, NV, NDIM, RS, CT, LIM, DIR, RT, CTT>, grid, SWEEP_THREADS, 0, s, a, g, seg, flat);
+  // sweeps side by side (launch_next in gp_kernels.cuh); with sums each sweep
+  // reads what the one before it wrote
+  if constexpr (PHYS != PHYS_RMHD && !sum_directions<PHYS, CTT>()) {
+    if (g.n <= kEarlyCells) {
+      launch(g.n, sweep_m_kernel<PHYS, NV, NDIM, RS, CT, LIM, DIR, true, RT, CTT>, grid, SWEEP_THREADS,
+             0, s, a, g, seg, flat);
+      post();
+      return;
+    }
+  }
+  launch(g.n, sweep_m_kernel<PHYS, NV, NDIM, RS, CT, LIM, DIR, false, RT, CTT>, grid, SWEEP_THREADS, 0,
+         s, a, g, seg, flat);
   post();
 }
 
@@ -165,7 +182,14 @@ static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, cudaStream_t 
     const int nseg = x_segments<PHYS, LIM, RT>(gd.nx, rows);
     dim3 grid((unsigned)(((long long)rows * nseg + wpb - 1) / wpb));
     pre();
-    launch(sweep_x_kernel<PHYS, NV, NDIM, RS, CT, LIM, RT, CTT>, grid, SWEEP_THREADS, 0, s, a, g, nseg);
+    // FP32 rows in one part keep their shuffles and carry (256^3: 546 us against
+    // 600 through shared memory, which is what parts of rows need)
+    if (sizeof(RT) == 4 && nseg == 1)
+      launch(gd.n, sweep_x_kernel<PHYS, NV, NDIM, RS, CT, LIM, sizeof(RT) == 4, RT, CTT>, grid,
+             SWEEP_THREADS, 0, s, a, g, nseg);
+    else
+      launch(gd.n, sweep_x_kernel<PHYS, NV, NDIM, RS, CT, LIM, false, RT, CTT>, grid, SWEEP_THREADS, 0, s,
+             a, g, nseg);
     post();
   }
   launch_m<PHYS, NV, NDIM, RS, CT, LIM, 1>(a, g, gd.nz, gd.ny, s, pre, post);
@@ -175,9 +199,9 @@ static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, cudaStream_t 
   if constexpr (PHYS != PHYS_HD) {
     pre();
     if constexpr (CT == CT_ARITH) {
-      launch(emf_arith_kernel<NDIM, RT, CTT>, nb, 256, 0, s, a, g);
+      launch(gd.n, emf_arith_kernel<NDIM, RT, CTT>, nb, 256, 0, s, a, g);
     } else if constexpr (CT == CT_CONTACT) {
-      launch(emf_contact_kernel<NDIM, RT, CTT>, nb, 256, 0, s, a, g);
+      launch(gd.n, emf_contact_kernel<NDIM, RT, CTT>, nb, 256, 0, s, a, g);
     } else if constexpr (NDIM == 3 && (sizeof(RT) == 8 || five_point<LIM>())) {  // plane-staged EMF
       using T = EmfTile<LIM, CTT>;
       cudaFuncSetAttribute(emf_tile_kernel<LIM, RT, CTT>,
@@ -188,7 +212,7 @@ static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, cudaStream_t 
       int sz = ET_SEGMENT;
       while (sz > 4 && cols * ((gd.nz + sz - 1) / sz) < 148LL * emf_tile_minb<RT>() * 4) sz /= 2;
       dim3 grid((gd.nx + ETX - 1) / ETX, (gd.ny + ETY - 1) / ETY, (gd.nz + sz - 1) / sz);
-      launch(emf_tile_kernel<LIM, RT, CTT>, grid, dim3(ETX, ETY), T::SMEM, s, a, g, sz);
+      launch(gd.n, emf_tile_kernel<LIM, RT, CTT>, grid, dim3(ETX, ETY), T::SMEM, s, a, g, sz);
     } else if constexpr (NDIM == 3) {  // mixed PLM/PPM: z-marching EMF, loads through L1
       // the longest segment (<= EMF_SEGMENT planes) that still gives about
       // four waves of blocks over 148 SMs (3 blocks per SM)
@@ -198,14 +222,14 @@ static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, cudaStream_t 
       while (sz > 4 && cols * ((gd.nz + sz - 1) / sz) < 148LL * 3 * 4) sz /= 2;
       dim3 grid((gd.nx + EMF_TX - 1) / EMF_TX, (gd.ny + EMF_TY - 1) / EMF_TY,
                 (gd.nz + sz - 1) / sz);
-      launch(emf_march_kernel<LIM, RT, CTT>, grid, dim3(EMF_TX, EMF_TY), 0, s, a, g, sz);
+      launch(gd.n, emf_march_kernel<LIM, RT, CTT>, grid, dim3(EMF_TX, EMF_TY), 0, s, a, g, sz);
     } else {
-      launch(emf_kernel<NDIM, LIM, RT, CTT>, nb, 256, 0, s, a, g);
+      launch(gd.n, emf_kernel<NDIM, LIM, RT, CTT>, nb, 256, 0, s, a, g);
     }
     post();
   }
   pre();
-  launch(finish_kernel<PHYS, NV, NDIM, CTT>, nb, 256, 0, s, a, g);
+  launch(gd.n, finish_kernel<PHYS, NV, NDIM, CTT>, nb, 256, 0, s, a, g);
   post();
 }
 

@@ -10,7 +10,6 @@
 // Riemann fluxes; the callers keep accumulation in FP64).
 #pragma once
 #include <cstdint>
-#include <type_traits>
 #include <cuda_runtime.h>
 
 #include "gp_exact.cuh"
@@ -541,7 +540,6 @@ __device__ __forceinline__ R mhd_hlld_line(const R* vl, const R* vr, R* flux, R 
   const R dsl = Sl - SM, dsr = Sr - SM;
   const R ysl = ar.inv_pos(-dsl), ysr = ar.inv_pos(dsr);
   const R rhosl = ar.quot_bpos(-rdl, -dsl, ysl), rhosr = ar.quot_bpos(rdr, dsr, ysr);
-  ar.densities(rhosl, rhosr);
   const R sqrL = ar.root(rhosl), sqrR = ar.root(rhosr);
   const R yqL = ar.inv_in(sqrL), yqR = ar.inv_in(sqrR);
   ar.check(Bx);
@@ -904,15 +902,16 @@ __device__ __noinline__ void mhd_hlld_call(R* io) {
   face_out(io, flux, ct, cmax);
 }
 
-// HLLD of both forms: the straight-line solver, and mhd_hlld where its flag is
-// set.
-template <int DIR, int CT, typename R>
-__device__ __forceinline__ R mhd_hlld_face(const R* vl, const R* vr, R* flux, R gamma, R ygm,
-                                           R Bn, CTFace<R>& ct) {
-  std::conditional_t<sizeof(R) == sizeof(double), FastArith, FloatArith> ar;
-  R cmax = mhd_hlld_line<DIR, CT>(vl, vr, flux, gamma, ygm, Bn, ct, ar);
-  if (ar.bad || ygm == R(0)) {
-    R io[18];
+// FP64 HLLD: the straight-line solver, and mhd_hlld where its flag is set.
+template <int DIR, int CT>
+__device__ __forceinline__ double mhd_hlld_fp64(const double* vl, const double* vr, double* flux,
+                                                double gamma, double ygm, double Bn,
+                                                CTFace<double>& ct) {
+  FastArith ar;
+  ar.bad = ygm == 0.0;
+  double cmax = mhd_hlld_line<DIR, CT>(vl, vr, flux, gamma, ygm, Bn, ct, ar);
+  if (ar.bad) {
+    double io[18];
     face_in(io, vl, vr, gamma, Bn);
     mhd_hlld_call<DIR, CT>(io);
     cmax = face_back(io, flux, ct);

@@ -18,6 +18,9 @@ __global__ void probe(const double* a, const double* b, double* out, double* ref
   } else if (op == 3) {
     out[i] = f.quot_pos(a[i], b[i], f.inv_pos(b[i]));
     ref[i] = a[i] / b[i];
+  } else if (op == 5) {
+    out[i] = f.div_any(a[i], b[i]);
+    ref[i] = a[i] / b[i];
   } else {
     out[i] = gp::fixed_quot(a[i], b[i], gp::fixed_inv(b[i]));
     ref[i] = a[i] / b[i];

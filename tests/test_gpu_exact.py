@@ -13,7 +13,7 @@ import pytest
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 HERE = os.path.dirname(os.path.abspath(__file__))
-DIV, INV, ROOT, QUOT_POS, FIXED = range(5)
+DIV, INV, ROOT, QUOT_POS, FIXED, DIV_ANY = range(6)
 
 
 @pytest.fixture(scope="module")
@@ -62,6 +62,8 @@ def test_random_arguments(probe, near):
         sign = torch.where(_random(n, 0, 2, 200 + seed) < 2, 1.0, -1.0).double()
         _same(*probe(a * sign, b, DIV), 0.0)
         _same(*probe(a, -b, DIV), 0.0)
+        _same(*probe(a * sign, b, DIV_ANY), 0.0)
+        _same(*probe(a, -b, DIV_ANY), 0.0)
         _same(*probe(a, b, INV), 0.0)
         _same(*probe(a, b, QUOT_POS), 0.0)
         _same(*probe(_random(n, -400, 400, 300 + seed, near), b, ROOT), 0.0)
@@ -76,6 +78,7 @@ def test_next_to_rounding_boundaries(probe):
     for k in (-2, -1, 0, 1, 2):   # dividends whose quotient is q to within an ulp or so
         a = ((q * b).view(torch.int64) + k).view(torch.float64)
         _same(*probe(a, b, DIV), 0.0)
+        _same(*probe(-a, b, DIV_ANY), 0.0)
         s = ((q * q).view(torch.int64) + k).view(torch.float64)   # roots next to q
         _same(*probe(s, b, ROOT), 0.0)
 
@@ -83,8 +86,9 @@ def test_next_to_rounding_boundaries(probe):
 def test_special_values(probe):
     tiny, inf, nan = 5e-324, float("inf"), float("nan")
     for a, b in ((0.0, 3.0), (-0.0, 3.0), (0.0, -3.0), (-0.0, -3.0)):
-        out, ref, bad = probe([a], [b], DIV)
-        assert not bad.any() and torch.equal(out.view(torch.int64), ref.view(torch.int64))
+        for op in (DIV, DIV_ANY):
+            out, ref, bad = probe([a], [b], op)
+            assert not bad.any() and torch.equal(out.view(torch.int64), ref.view(torch.int64))
     ones = np.nextafter(2.0, 0.0)
     for a in (1.0, ones, np.nextafter(ones, 0.0), 3.0, -ones):
         for b in (ones, ones / 2, -ones, np.nextafter(ones, 0.0)):
@@ -95,8 +99,7 @@ def test_special_values(probe):
     for a, b in ((1.0, 0.0), (1.0, tiny), (1.0, inf), (1.0, nan), (tiny, 1.0),
                  (1e-320, 3.0), (inf, 1.0), (nan, 1.0), (1e-250, 1.0), (1e250, 1.0),
                  (1.0, 1e70), (1.0, 1e-70)):
-        out, ref, bad = probe([a], [b], DIV)
-        assert bad.all()
+        assert probe([a], [b], DIV)[2].all() and probe([a], [b], DIV_ANY)[2].all()
         out, ref, bad = probe([a], [b], FIXED)    # falls back by itself
         assert torch.equal(out.view(torch.int64), ref.view(torch.int64)) or np.isnan(a + b)
     for a in (0.0, -0.0, -1.0, tiny, 1e-320, inf, nan, 1e-130, 1e130):

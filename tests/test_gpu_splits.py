@@ -80,3 +80,22 @@ def test_zeros(ndim):
         st.V[4] = field
         st.Bs = [np.full_like(b, field if d == 0 else 0.0) for d, b in enumerate(st.Bs)]
         check(st, nsteps=3)
+
+
+@pytest.mark.parametrize("precision", [api.FP64, api.MIXED])
+@pytest.mark.parametrize("n", [(64, 48), (333, 31), (40, 36, 30)])
+@pytest.mark.parametrize("physics", ["hd", "mhd"])
+def test_overlapped_sweeps_match_serialized_launches(physics, n, precision):
+    """The sweeps of a small grid's stage run side by side; profiling records an
+    event around each launch, which puts them back in a row."""
+    gen = ics.hd_turbulence if physics == "hd" else \
+        (ics.mhd2d_turbulence if len(n) == 2 else ics.mhd3d_turbulence)
+    st = gen(n=n, seed=11)
+    hd = physics == "hd"
+    sch = api.Scheme(physics=st.physics, riemann="hllc" if hd else "hlld",
+                     ct_emf="uct_hll" if hd else "uct_hlld", gamma=st.gamma, precision=precision)
+    a, b = api.Solver.from_state(st, sch), api.Solver.from_state(st, sch)
+    a.run(40, 1e-4)
+    b.profile(40, 1e-4)
+    for x, y in zip(a.download(), b.download()):
+        np.testing.assert_array_equal(np.asarray(x), np.asarray(y))
