@@ -809,7 +809,7 @@ int gp_create(const gp_grid_desc* grid, const gp_scheme* scheme, void* stream,
         fills += (side & 1) + (scheme->physics == GP_HD ? 0 : 1);
       else
         fills += scheme->physics == GP_HD ? 1 : 2;
-    h->launches_per_step = scheme->rk_stages * (gp::stage_launch_count(h->key) + fills) + 1;
+    h->launches_per_step = scheme->rk_stages * (gp::stage_launches(h->key, h->mixed) + fills) + 1;
   }
   if (h->padded) {  // padding cells start finite
     cudaMemsetAsync(h->V, 0, cell * h->nvar, h->stream);

@@ -89,11 +89,13 @@ __device__ __forceinline__ int gidx(int i, int n, unsigned outflow, int d) {
   return i;
 }
 
+// An ordinary (coherent) load: V is written by the kernel before, which may
+// still run when this one's blocks are placed (step_order), so the read-only
+// path, which needs V constant for the kernel's whole life, is not open.
 template <int NV, typename R>
-__device__ __forceinline__ void load_cell(const double* __restrict__ V, long long n,
-                                          long long c, R* v) {
+__device__ __forceinline__ void load_cell(const double* V, long long n, long long c, R* v) {
 #pragma unroll
-  for (int nv = 0; nv < NV; nv++) v[nv] = (R)__ldg(V + nv * n + c);
+  for (int nv = 0; nv < NV; nv++) v[nv] = (R)V[nv * n + c];
 }
 
 // Asynchronous global->shared copies (cp.async, per thread, 8 bytes): the
@@ -113,32 +115,14 @@ __device__ __forceinline__ void cp_async_wait0() {
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
-// Programmatic dependent launch.  launch_next lets the next kernel's blocks be
-// placed once all blocks of this one have called it; wait_before returns when
-// every kernel launched before this one has completed and its writes are
-// visible.  A kernel calls launch_next and wait_before first of all.  With
-// OVERLAP the sweeps of a stage, which do not read one another's results, run
-// side by side:
-//   * the x-sweep calls wait_before first, so that the kernel it lets in
-//     starts after the state it needs is complete;
-//   * the y and z sweeps start at once and call wait_before last, so that
-//     their own completion means the sweep's before them.  (A kernel of its
-//     own: the call at the end cost the large grids' one 64 bytes of spills
-//     and 3%.)
-// Small grids are bound by the launches' latency and by each sweep's own chain
-// (2-D MHD 64^2: step 82 -> 72 us with the launches, 63 with the sweeps
-// overlapped; 256^2, ten steps: 808 -> 706 -> 684; 61x47x53, five steps: 941 ->
-// 905 -> 831).  The host does both up to 2^20 cells (kEarlyCells) and does not
-// overlap RMHD: RMHD 90x72x60 lost 12% (two long codes in one instruction cache).
-__device__ __forceinline__ void launch_next() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void wait_before() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
+// Programmatic dependent launch.  The first instruction lets the next kernel's
+// blocks be placed once all blocks of this one have executed it, the second
+// returns when every kernel launched before this one has completed and its
+// writes are visible.  Every kernel of a step calls this before it reads or
+// writes global memory, so only the launches overlap, not the work.
 __device__ __forceinline__ void step_order() {
-  launch_next();
-  wait_before();
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 #ifndef GP_SWEEP_MINB
@@ -147,19 +131,28 @@ __device__ __forceinline__ void step_order() {
 constexpr int SWEEP_THREADS = 128;
 
 // Resident 128-thread blocks per SM the sweep kernels are compiled for
-// (register budget 65536 / (128 * blocks)), measured at 256^3 on 3-D MHD:
-// FP64 x-sweep 3 (168 registers; at 4 1084 -> 1142 us), FP64 y/z sweeps 4 (128;
-// at 3 the same), mixed form 5 (102; at 6 x 568 -> 779 us).  The relativistic
-// solver's long code runs at 2, fewer warps walking it at once (192^3 FP64 y/z
-// 3617/4335 us at 3, 3152/3885 at 2); its mixed y/z sweeps stay at 3, which
-// fits small grids' waves better (90x72x60: 260 against 314 us).
+// (register budget 65536 / (128 * blocks)).
+//
+// All sweeps in one kernel (sweeps_kernel: MHD, mixed HD).  FP64 at 3 (168
+// registers): 1000^2 four steps 1755 us, 100^3 2847; at 2, without spills, 1816
+// and 2972 (256^2 ten steps 643 and 608).  FP32 MHD at 4 (126): 333x171 ten steps
+// 505 us, 64^3 PPM four steps 782, 200^3 12723; at 5 518, 822 and 12628.  FP32 HD
+// at 5: 384^2 four steps 174 us (at 4 183).
+template <int PHYS, typename R>
+constexpr int sweeps_minb() {
+  return sizeof(R) == 8 ? 3 : (PHYS == PHYS_MHD ? 4 : 5);
+}
+// One kernel a sweep (RMHD, FP64 HD): HD x 3, y/z 4.  The relativistic solver's
+// long code runs at 2, fewer warps walking it at once (192^3 FP64 y/z 3617/4335 us
+// at 3, 3152/3885 at 2); its mixed y/z sweeps stay at 3, which fits small grids'
+// waves better (90x72x60: 260 against 314 us).
 template <int PHYS, typename R>
 constexpr int sweep_x_minb() {
-  return PHYS == PHYS_RMHD ? 2 : (sizeof(R) == 4 ? 5 : 3);
+  return PHYS == PHYS_RMHD ? 2 : 3;
 }
 template <int PHYS, typename R>
 constexpr int sweep_m_minb() {
-  return PHYS == PHYS_RMHD ? (sizeof(R) == 4 ? 3 : 2) : (sizeof(R) == 4 ? 5 : 4);
+  return PHYS == PHYS_RMHD ? (sizeof(R) == 4 ? 3 : 2) : 4;
 }
 
 // whether the single-grid kernels add the directions' flux differences up in
@@ -325,6 +318,12 @@ constexpr int sweep_m_stage_doubles() {
   return ((LIM == LIM_PPM ? 5 * NV + 2 : five_point<LIM>() ? 2 * (NV + 1) : 4 * NV + 2) +
           (SUM ? 2 * sum_slots<NV>() : 0)) *
          SWEEP_THREADS;
+}
+
+// FP32 rows in one part have a form of their own (sweep_x_row_f32)
+template <int LIM, typename R>
+constexpr bool whole_row_form() {
+  return sizeof(R) == 4 && LIM != LIM_PPM && !five_point<LIM>();
 }
 
 // Piecewise parabolic x-row (one warp per row).  Lane l of a chunk owns
@@ -1035,22 +1034,28 @@ __device__ __forceinline__ void sweep_x_row(const StageArgs<CTT>& a, const Grid3
   if (err) atomicOr(a.err, err);
 }
 
-// WHOLE: one row a warp, FP32 (the host's x_segments gave one part)
+// Block `block` of the x-sweep, rows in nseg parts.  WHOLE: sweep_x_row_f32
+// (nseg = 1).
+template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, bool WHOLE, typename R, typename CTT>
+__device__ __forceinline__ void sweep_x_block(const StageArgs<CTT>& a, const Grid3& g, int nseg,
+                                              int block, double* stg) {
+  const int w = block * (SWEEP_THREADS / 32) + (threadIdx.x >> 5);
+  if constexpr (WHOLE) {
+    sweep_x_row_f32<PHYS, NV, NDIM, RS, CT, LIM, R, CTT>(a, g, w, stg, threadIdx.x);
+  } else {
+    const int row = w / nseg, q = w - row * nseg;
+    sweep_x_row<PHYS, NV, NDIM, RS, CT, LIM, R, CTT>(a, g, row, (int)((long long)g.nx * q / nseg),
+                                                     (int)((long long)g.nx * (q + 1) / nseg), stg,
+                                                     threadIdx.x);
+  }
+}
+
 template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, bool WHOLE, typename R, typename CTT>
 __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_x_minb<PHYS, R>()))
     sweep_x_kernel(StageArgs<CTT> a, Grid3 g, int nseg) {
   __shared__ double stg[sweep_x_stage_doubles<NV, LIM>()];
-  wait_before();
-  launch_next();
-  const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if constexpr (WHOLE && LIM != LIM_PPM && !five_point<LIM>()) {
-    sweep_x_row_f32<PHYS, NV, NDIM, RS, CT, LIM, R, CTT>(a, g, w, stg, threadIdx.x);
-    return;
-  }
-  const int row = w / nseg, q = w - row * nseg;
-  sweep_x_row<PHYS, NV, NDIM, RS, CT, LIM, R, CTT>(a, g, row, (int)((long long)g.nx * q / nseg),
-                                                   (int)((long long)g.nx * (q + 1) / nseg), stg,
-                                                   threadIdx.x);
+  step_order();
+  sweep_x_block<PHYS, NV, NDIM, RS, CT, LIM, WHOLE, R, CTT>(a, g, nseg, blockIdx.x, stg);
 }
 
 // ---------------------------------------------------------------------
@@ -1561,31 +1566,33 @@ __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3
   if (err) atomicOr(a.err, err);
 }
 
-// t is the transverse index (k for DIR=1, j for DIR=2).  Grid (x-blocks,
-// t * nseg + seg), the block's columns sharing one t; with `flat` (nx not a
-// multiple of the block) a 1-D grid of (column block cb, segment) pairs,
-// segments innermost, with the (x, t) columns numbered together (col = cb *
-// SWEEP_THREADS + thread, i = col % nx, t = col / nx), so that no block is
-// part-empty.
-template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, bool OVERLAP, typename R,
-          typename CTT>
+// Thread's column i, transverse index t (k for DIR=1, j for DIR=2) and segment in
+// block `block` of a y or z sweep over nt transverse positions: (column block,
+// segment) pairs, segments innermost, with the (x, t) columns numbered together
+// (col = column block * SWEEP_THREADS + thread, i = col % nx, t = col / nx), so
+// that no block is part-empty whatever nx is.
+__device__ __forceinline__ void flat_column(int nx, int nt, unsigned nseg, unsigned block, int& i,
+                                            int& t, int& seg) {
+  seg = (int)(block % nseg);
+  const long long col = (long long)(block / nseg) * SWEEP_THREADS + (int)threadIdx.x;
+  t = (int)(col / nx);
+  i = (int)(col - (long long)t * nx);
+  if (t >= nt) i = nx;   // past the last column: the thread stays idle
+}
+
+// One y or z sweep.  Grid (x-blocks, t * nseg + seg), the block's columns sharing
+// one t; with `flat` (nx not a multiple of the block) flat_column's numbering.
+template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, typename R, typename CTT>
 __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_m_minb<PHYS, R>()))
     sweep_m_kernel(StageArgs<CTT> a, Grid3 g, int S, bool flat) {
   constexpr bool SUM = sum_directions<PHYS, CTT>();
   __shared__ double stg[sweep_m_stage_doubles<NV, LIM, SUM>()];
-  launch_next();
-  if (!OVERLAP) wait_before();
+  step_order();
   const int nd = (DIR == 1) ? g.ny : g.nz;
   const int nseg = (nd + S - 1) / S;
   int i, t, seg;
   if (flat) {
-    const int nt = (DIR == 1) ? g.nz : g.ny;
-    seg = (int)(blockIdx.x % (unsigned)nseg);
-    const long long col =
-        (long long)(blockIdx.x / (unsigned)nseg) * SWEEP_THREADS + (int)threadIdx.x;
-    t = (int)(col / g.nx);
-    i = (int)(col - (long long)t * g.nx);
-    if (t >= nt) i = g.nx;   // past the last column: the thread stays idle
+    flat_column(g.nx, (DIR == 1) ? g.nz : g.ny, nseg, blockIdx.x, i, t, seg);
   } else {
     i = blockIdx.x * SWEEP_THREADS + threadIdx.x;
     t = blockIdx.y / nseg;
@@ -1593,7 +1600,51 @@ __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_m_minb<PHYS, R>()))
   }
   sweep_m_col<PHYS, NV, NDIM, RS, CT, LIM, DIR, SUM, R, CTT>(a, g, i, t, seg, S, stg,
                                                              threadIdx.x);
-  if (OVERLAP) wait_before();
+}
+
+// All sweeps of a stage in one launch: the directions write arrays of their own
+// and none reads what another wrote, so their blocks run side by side in any order.
+// Small grids are bound by the launches' latency and by each sweep's own chain, and
+// on large ones a sweep's last wave is filled by the next one's blocks.  Against one
+// launch a sweep: 2-D MHD 64^2 step 74 -> 64 us, 256^2 ten steps 719 -> 643,
+// 61x47x53 five steps 917 -> 735; four steps of 112^3 3884 -> 3611, 160^3 10156 ->
+// 9567, 200^3 20486 -> 19867, mixed 126^3 3528 -> 3311, 160^3 6457 -> 6318, 200^3 PPM
+// + RK3 24321 -> 24159, HD mixed 160^3 2814 -> 2687; 256^3 blast step 9988 -> 9676,
+// mixed 6100 -> 6097.  RMHD keeps one launch a sweep (90x72x60 lost 12%: two long
+// codes in one instruction cache), and so do the forms whose sweeps add up in one
+// array.
+// Blocks [0, nb[0]) sweep z, the next nb[1] y, the rest x; `first` is the number of
+// the launch's first block, so that one direction can be launched (and timed) alone.
+struct SweepSplit {
+  int first;
+  int xseg, len[2];  // parts of an x-row, march lengths (y, z)
+  int nb[2];         // blocks (z, y)
+};
+
+template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, bool WHOLE, typename R, typename CTT>
+__global__ void __launch_bounds__(SWEEP_THREADS, (sweeps_minb<PHYS, R>()))
+    sweeps_kernel(StageArgs<CTT> a, Grid3 g, SweepSplit sp) {
+  constexpr int nx = sweep_x_stage_doubles<NV, LIM>();
+  constexpr int nm = sweep_m_stage_doubles<NV, LIM>();
+  __shared__ double stg[nx > nm ? nx : nm];
+  step_order();
+  int b = sp.first + blockIdx.x, i, t, seg;
+  if constexpr (NDIM == 3) {
+    if (b < sp.nb[0]) {
+      flat_column(g.nx, g.ny, (unsigned)((g.nz + sp.len[1] - 1) / sp.len[1]), b, i, t, seg);
+      sweep_m_col<PHYS, NV, NDIM, RS, CT, LIM, 2, false, R, CTT>(a, g, i, t, seg, sp.len[1], stg,
+                                                                 threadIdx.x);
+      return;
+    }
+  }
+  b -= sp.nb[0];
+  if (b < sp.nb[1]) {
+    flat_column(g.nx, g.nz, (unsigned)((g.ny + sp.len[0] - 1) / sp.len[0]), b, i, t, seg);
+    sweep_m_col<PHYS, NV, NDIM, RS, CT, LIM, 1, false, R, CTT>(a, g, i, t, seg, sp.len[0], stg,
+                                                               threadIdx.x);
+    return;
+  }
+  sweep_x_block<PHYS, NV, NDIM, RS, CT, LIM, WHOLE, R, CTT>(a, g, sp.xseg, b - sp.nb[1], stg);
 }
 
 // ---------------------------------------------------------------------

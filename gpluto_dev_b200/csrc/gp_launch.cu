@@ -68,9 +68,16 @@ static StageArgs<CTT> make_args(const StageDesc& d) {
   return a;
 }
 
-// Grids up to this many cells are launched early and overlap their sweeps: at
-// 256^3 early launches cost the mixed step 1.5% and the FP64 step 1%.
+// Grids up to this many cells are launched early.  Above it the launches' latency is
+// hidden anyway and it depends on the form (four steps, late -> early): MHD FP64 126^3
+// 5394 -> 5424 us, 160^3 10156 -> 10250, RMHD 112^3 22265 -> 22448, HD 126^3 1967 ->
+// 1933, MHD mixed 126^3 3528 -> 3483; 256^3 MHD one step FP64 +1%, mixed +1.5%.
 constexpr long long kEarlyCells = 1LL << 20;
+
+// Forms that sweep all directions in one launch (sweeps_kernel)
+constexpr bool one_sweep_launch(int physics, bool mixed) {
+  return physics == PHYS_MHD || (physics == PHYS_HD && mixed);
+}
 
 // Launch in stream order, on a grid of at most kEarlyCells cells with its blocks
 // placed while the kernel before drains (step_order)
@@ -95,10 +102,10 @@ static void launch(long long cells, void (*k)(K...), dim3 grid, dim3 block, size
 // periodic row needs no extra face.  The count with the fewest (waves of
 // resident warps) x (chunks, + 1 for the start-up) is taken: one for grids
 // that fill the SMs with whole rows.
-template <int PHYS, int LIM, typename R>
-static int x_segments(int nx, long long rows) {
+template <int LIM>
+static int x_segments(int nx, long long rows, int blocks_per_sm) {
   if (LIM == LIM_PPM || five_point<LIM>()) return 1;
-  const long long resident = 148LL * sweep_x_minb<PHYS, R>() * (SWEEP_THREADS / 32);
+  const long long resident = 148LL * blocks_per_sm * (SWEEP_THREADS / 32);
   auto cost = [&](int nseg, int chunks) {
     return (rows * nseg + resident - 1) / resident * (chunks + 1);
   };
@@ -119,9 +126,8 @@ static int x_segments(int nx, long long rows) {
 // marched, + 2 for the start-up and the face at the end).  A last wave that
 // fills few SMs costs a whole wave, and a grid that does not fill them takes
 // the shortest march.
-template <int PHYS, typename R>
-static int march_length(long long cols, int nd) {
-  const long long resident = 148LL * sweep_m_minb<PHYS, R>();
+static int march_length(long long cols, int nd, int blocks_per_sm) {
+  const long long resident = 148LL * blocks_per_sm;
   int best = 1;
   long long c = 0;
   for (int len = 1; len <= nd && len <= 128; len++) {
@@ -136,31 +142,63 @@ static int march_length(long long cols, int nd) {
 }
 
 // y or z sweep over nt transverse positions of nd cells: grid (x-blocks,
-// transverse index x pencil segments); when nx is not a multiple of the
-// block, a 1-D grid over (x, transverse) columns numbered together, so that
-// no block is part-empty.
-template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, typename F1, typename F2>
-static void launch_m(const StageArgs<CTT>& a, const Grid3& g, int nt, int nd, cudaStream_t s,
-                     F1& pre, F2& post) {
+// transverse index x pencil segments), flat when nx is not a multiple of the
+// block (sweep_m_kernel)
+template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR>
+static void launch_m(const StageArgs<CTT>& a, const Grid3& g, int nt, int nd, cudaStream_t s) {
   const long long cols = ((long long)g.nx * nt + SWEEP_THREADS - 1) / SWEEP_THREADS;
-  const int seg = march_length<PHYS, RT>(cols, nd);
+  const int seg = march_length(cols, nd, sweep_m_minb<PHYS, RT>());
   const int nseg = (nd + seg - 1) / seg;
-  pre();
   const bool flat = g.nx % SWEEP_THREADS != 0 || (long long)nt * nseg > 65535;
   const dim3 grid = flat ? dim3((unsigned)(cols * nseg)) : dim3(g.nx / SWEEP_THREADS, nt * nseg);
-  // sweeps side by side (launch_next in gp_kernels.cuh); with sums each sweep
-  // reads what the one before it wrote
-  if constexpr (PHYS != PHYS_RMHD && !sum_directions<PHYS, CTT>()) {
-    if (g.n <= kEarlyCells) {
-      launch(g.n, sweep_m_kernel<PHYS, NV, NDIM, RS, CT, LIM, DIR, true, RT, CTT>, grid, SWEEP_THREADS,
-             0, s, a, g, seg, flat);
-      post();
-      return;
-    }
+  launch(g.n, sweep_m_kernel<PHYS, NV, NDIM, RS, CT, LIM, DIR, RT, CTT>, grid, SWEEP_THREADS, 0, s,
+         a, g, seg, flat);
+}
+
+// blocks of an x-sweep whose rows are in nseg parts
+static unsigned x_blocks(long long rows, int nseg) {
+  const int wpb = SWEEP_THREADS / 32;
+  return (unsigned)((rows * nseg + wpb - 1) / wpb);
+}
+
+// The sweeps of a stage in one launch; with `each` in one launch a direction of the
+// same kernel (x, y, z), so that profiled steps keep the bits.
+template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, typename F1, typename F2>
+static void launch_sweeps(const StageArgs<CTT>& a, const Grid3& g, cudaStream_t s, bool each,
+                          F1& pre, F2& post) {
+  constexpr int per_sm = sweeps_minb<PHYS, RT>();
+  const long long rows = (long long)g.ny * g.nz;
+  SweepSplit sp = {};
+  sp.xseg = x_segments<LIM>(g.nx, rows, per_sm);
+  const long long cy = ((long long)g.nx * g.nz + SWEEP_THREADS - 1) / SWEEP_THREADS;
+  sp.len[0] = march_length(cy, g.ny, per_sm);
+  sp.nb[1] = (int)(cy * ((g.ny + sp.len[0] - 1) / sp.len[0]));
+  if (NDIM == 3) {
+    const long long cz = ((long long)g.nx * g.ny + SWEEP_THREADS - 1) / SWEEP_THREADS;
+    sp.len[1] = march_length(cz, g.nz, per_sm);
+    sp.nb[0] = (int)(cz * ((g.nz + sp.len[1] - 1) / sp.len[1]));
   }
-  launch(g.n, sweep_m_kernel<PHYS, NV, NDIM, RS, CT, LIM, DIR, false, RT, CTT>, grid, SWEEP_THREADS, 0,
-         s, a, g, seg, flat);
-  post();
+  const unsigned nbx = x_blocks(rows, sp.xseg);
+  auto blocks = [&](unsigned first, unsigned count) {
+    sp.first = (int)first;
+    pre();
+    // FP32 rows in one part keep their shuffles and carry (256^3: 546 us against
+    // 600 through shared memory, which is what parts of rows need)
+    if (whole_row_form<LIM, RT>() && sp.xseg == 1)
+      launch(g.n, sweeps_kernel<PHYS, NV, NDIM, RS, CT, LIM, whole_row_form<LIM, RT>(), RT, CTT>,
+             count, SWEEP_THREADS, 0, s, a, g, sp);
+    else
+      launch(g.n, sweeps_kernel<PHYS, NV, NDIM, RS, CT, LIM, false, RT, CTT>, count, SWEEP_THREADS,
+             0, s, a, g, sp);
+    post();
+  };
+  if (!each) {
+    blocks(0, sp.nb[0] + sp.nb[1] + nbx);
+    return;
+  }
+  blocks(sp.nb[0] + sp.nb[1], nbx);
+  blocks(sp.nb[0], sp.nb[1]);
+  if (NDIM == 3) blocks(0, sp.nb[0]);
 }
 
 template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM>
@@ -176,25 +214,30 @@ static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, cudaStream_t 
   int kidx = 0;
   auto pre = [&]() { if (ev) cudaEventRecord(ev[2 * kidx], s); };
   auto post = [&]() { if (ev) cudaEventRecord(ev[2 * kidx + 1], s); kidx++; };
-  {
+  if constexpr (one_sweep_launch(PHYS, sizeof(RT) == 4)) {
+    static_assert(!sum_directions<PHYS, CTT>(), "the sweeps read one another's sums");
+    launch_sweeps<PHYS, NV, NDIM, RS, CT, LIM>(a, g, s, ev != nullptr, pre, post);
+  } else {
     const int rows = gd.ny * gd.nz;
-    const int wpb = SWEEP_THREADS / 32;
-    const int nseg = x_segments<PHYS, LIM, RT>(gd.nx, rows);
-    dim3 grid((unsigned)(((long long)rows * nseg + wpb - 1) / wpb));
+    const int nseg = x_segments<LIM>(gd.nx, rows, sweep_x_minb<PHYS, RT>());
+    const unsigned grid = x_blocks(rows, nseg);
     pre();
-    // FP32 rows in one part keep their shuffles and carry (256^3: 546 us against
-    // 600 through shared memory, which is what parts of rows need)
-    if (sizeof(RT) == 4 && nseg == 1)
-      launch(gd.n, sweep_x_kernel<PHYS, NV, NDIM, RS, CT, LIM, sizeof(RT) == 4, RT, CTT>, grid,
-             SWEEP_THREADS, 0, s, a, g, nseg);
+    if (whole_row_form<LIM, RT>() && nseg == 1)
+      launch(gd.n, sweep_x_kernel<PHYS, NV, NDIM, RS, CT, LIM, whole_row_form<LIM, RT>(), RT, CTT>,
+             grid, SWEEP_THREADS, 0, s, a, g, nseg);
     else
-      launch(gd.n, sweep_x_kernel<PHYS, NV, NDIM, RS, CT, LIM, false, RT, CTT>, grid, SWEEP_THREADS, 0, s,
-             a, g, nseg);
+      launch(gd.n, sweep_x_kernel<PHYS, NV, NDIM, RS, CT, LIM, false, RT, CTT>, grid, SWEEP_THREADS,
+             0, s, a, g, nseg);
     post();
+    pre();
+    launch_m<PHYS, NV, NDIM, RS, CT, LIM, 1>(a, g, gd.nz, gd.ny, s);
+    post();
+    if constexpr (NDIM == 3) {
+      pre();
+      launch_m<PHYS, NV, NDIM, RS, CT, LIM, 2>(a, g, gd.ny, gd.nz, s);
+      post();
+    }
   }
-  launch_m<PHYS, NV, NDIM, RS, CT, LIM, 1>(a, g, gd.nz, gd.ny, s, pre, post);
-  if constexpr (NDIM == 3) 
-    launch_m<PHYS, NV, NDIM, RS, CT, LIM, 2>(a, g, gd.ny, gd.nz, s, pre, post);
   const unsigned nb = (unsigned)((gd.n + 255) / 256);
   if constexpr (PHYS != PHYS_HD) {
     pre();
@@ -353,6 +396,10 @@ int stage_launch_count(const SchemeKey& k) {
   int c = 1 + (k.ndim == 3 ? 2 : 1) + 1;  // sweeps + finish
   if (k.physics != PHYS_HD) c += 1;       // emf
   return c;
+}
+
+int stage_launches(const SchemeKey& k, bool mixed) {
+  return stage_launch_count(k) - (one_sweep_launch(k.physics, mixed) ? k.ndim - 1 : 0);
 }
 
 const char* stage_kernel_name(const SchemeKey& k, int idx) {

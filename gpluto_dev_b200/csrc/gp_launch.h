@@ -55,8 +55,11 @@ int launch_prim2cons(int physics, const double* V, double* U, long long n, doubl
 // Sets the text returned by gp_last_error on this thread; returns `code`.
 int set_last_error(int code, const char* msg);
 
-// Number of kernel launches one stage issues for this scheme, and their names.
+// Number of kernel launches one stage issues for this scheme with events between
+// them, and their names; and the number without events (MHD and mixed HD sweep all
+// directions in one launch).
 int stage_launch_count(const SchemeKey& k);
+int stage_launches(const SchemeKey& k, bool mixed);
 const char* stage_kernel_name(const SchemeKey& k, int idx);
 
 }  // namespace gp

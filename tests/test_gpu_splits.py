@@ -86,8 +86,9 @@ def test_zeros(ndim):
 @pytest.mark.parametrize("n", [(64, 48), (333, 31), (40, 36, 30)])
 @pytest.mark.parametrize("physics", ["hd", "mhd"])
 def test_overlapped_sweeps_match_serialized_launches(physics, n, precision):
-    """The sweeps of a small grid's stage run side by side; profiling records an
-    event around each launch, which puts them back in a row."""
+    """MHD and mixed HD sweep all directions in one launch; profiling sweeps them in
+    a launch each with events around it, which puts them in a row.  FP64 HD has a
+    launch a sweep either way: there the events only undo the early launches."""
     gen = ics.hd_turbulence if physics == "hd" else \
         (ics.mhd2d_turbulence if len(n) == 2 else ics.mhd3d_turbulence)
     st = gen(n=n, seed=11)
