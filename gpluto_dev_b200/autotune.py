@@ -13,7 +13,8 @@ and, for the whole batch, the number of blocks of the persistent launch.
 
 The search is coordinate descent on the live batch: every trial times a few
 graph-replayed steps of all slots (host clock around advance + wait, best of
-``reps``), one parameter of one bin at a time, starting from the defaults.
+``reps``), one parameter of one bin at a time, starting from the library's own
+choice (0, made from all that the batch holds), which is also a candidate.
 Results do not depend on the tile shapes (the batch tests check this), so
 tuning on the grids that will be run is safe; the steps it takes count
 against the slots' budgets, so tune a copy or a sample.
@@ -31,8 +32,8 @@ import time
 
 from . import batch as gb
 
-SEGS = (8, 16, 32, 64)
-CPTS = (1, 2, 4, 8)
+SEGS = (0, 4, 8, 16, 32, 64)     # 0: the library's choice
+CPTS = (0, 1, 2, 4, 8, 16)
 CTAS_PER_SM = (1, 2, 3)
 NUM_SMS = 148
 
@@ -41,11 +42,12 @@ EDGES = (0, 1 << 13, 1 << 15, 1 << 17, 1 << 62)
 
 
 def default_table() -> dict:
+    """A table that leaves every shape to the library."""
     bins, shapes = [], []
     for ndim in (2, 3):
         for lo, hi in zip(EDGES[:-1], EDGES[1:]):
             bins.append([ndim, lo, hi])
-            shapes.append([32, 2])
+            shapes.append([0, 0])
     return {"bins": bins, "shapes": shapes, "ctas_per_sm": 0}
 
 
