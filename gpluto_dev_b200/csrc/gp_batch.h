@@ -99,9 +99,9 @@ __device__ void batch_cell_tile_mixed(const BatchSlot& s, const BatchTile& t, in
 
 // Shared memory a block needs (largest staging area of any phase).
 constexpr int batch_smem_bytes() {
-  return (int)sizeof(double) * (sweep_x_stage_doubles<8>() > sweep_m_stage_doubles<8>()
-                                    ? sweep_x_stage_doubles<8>()
-                                    : sweep_m_stage_doubles<8>());
+  constexpr int x = sweep_x_stage_doubles<8, LIM_MC, double, false>();
+  constexpr int m = sweep_m_stage_doubles<8, LIM_MC, double>();
+  return (int)sizeof(double) * (x > m ? x : m);
 }
 
 }  // namespace gp

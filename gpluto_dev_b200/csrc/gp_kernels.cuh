@@ -301,25 +301,30 @@ struct XRow {
   static constexpr int F0 = F + (NV + 1) * 33;       // [NV + 1] those of the row's first face
   static constexpr int SIZE = F0 + NV + 1;
 };
-template <int NV, int LIM = LIM_MC>
+template <int NV, int LIM, typename R, bool WHOLE>
 constexpr int sweep_x_stage_doubles() {
   return (LIM == LIM_PPM || five_point<LIM>())
              ? 2 * (2 * NV + 1) * SWEEP_THREADS + 2 * (SWEEP_THREADS / 32) * NV
-             : XRow<NV>::SIZE * (SWEEP_THREADS / 32);  // FP32: 2 * (2 * NV + 1) * 128 of them
+         : WHOLE ? 2 * (2 * NV + 1) * SWEEP_THREADS  // sweep_x_row_f32
+                 : XRow<NV>::SIZE * (SWEEP_THREADS / 32);
 }
-// y/z sweeps: a ring of four cells and two face fields per thread (PLM,
-// LimO3, WENO3), five cells (PPM), two cells and face fields otherwise
 // values SumStage keeps of a cell: flux differences (at most 6 with a field in
 // two directions) and the inverse-dt term
 template <int NV>
 constexpr int sum_slots() { return NV == 8 ? 7 : NV + 1; }
-template <int NV, int LIM = LIM_MC, bool SUM = false>
+// y/z sweeps, per thread: FP64 a ring of four cells and two face fields (PLM,
+// LimO3, WENO3) or of five cells (PPM); MP5, WENO-Z and every FP32 form, whose
+// cells stay in a register window, two cells and two face fields.  What the FP32
+// kernels leave goes to L1 (against the FP64 rings' sizes: PPM + RK3 126^3 four
+// steps 6420 -> 6371 us, RMHD 180^3 79.5 -> 79.3 ms, PLM the same).
+template <int NV, int LIM, typename R, bool SUM = false>
 constexpr int sweep_m_stage_doubles() {
-  return ((LIM == LIM_PPM ? 5 * NV + 2 : five_point<LIM>() ? 2 * (NV + 1) : 4 * NV + 2) +
+  return ((sizeof(R) == 4 || five_point<LIM>() ? 2 * (NV + 1)
+           : LIM == LIM_PPM                    ? 5 * NV + 2
+                                               : 4 * NV + 2) +
           (SUM ? 2 * sum_slots<NV>() : 0)) *
          SWEEP_THREADS;
 }
-
 // FP32 rows in one part have a form of their own (sweep_x_row_f32)
 template <int LIM, typename R>
 constexpr bool whole_row_form() {
@@ -873,7 +878,7 @@ __device__ __forceinline__ void sweep_x_row_f32(const StageArgs<CTT>& a, const G
 // A whole periodic row solves faces 0 .. nx-1 and keeps face 0 for its last
 // cell; a part of a row (s0 > 0 or s1 < nx, used when whole rows would leave
 // SMs idle) or a row with an outflow high side also solves face s1.
-// `stg_` is the block's staging area (sweep_x_stage_doubles<NV, LIM>()
+// `stg_` is the block's staging area (sweep_x_stage_doubles<NV, LIM, R, false>()
 // doubles of shared memory), `tid` the thread's index in its 128-thread block.
 template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, typename R, typename CTT>
 __device__ __forceinline__ void sweep_x_row(const StageArgs<CTT>& a, const Grid3& g, int row,
@@ -1053,7 +1058,7 @@ __device__ __forceinline__ void sweep_x_block(const StageArgs<CTT>& a, const Gri
 template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, bool WHOLE, typename R, typename CTT>
 __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_x_minb<PHYS, R>()))
     sweep_x_kernel(StageArgs<CTT> a, Grid3 g, int nseg) {
-  __shared__ double stg[sweep_x_stage_doubles<NV, LIM>()];
+  __shared__ double stg[sweep_x_stage_doubles<NV, LIM, R, WHOLE>()];
   step_order();
   sweep_x_block<PHYS, NV, NDIM, RS, CT, LIM, WHOLE, R, CTT>(a, g, nseg, blockIdx.x, stg);
 }
@@ -1110,8 +1115,11 @@ template <int PHYS, int NV, int NDIM, int RS, int CT, int DIR, bool SUM, typenam
 __device__ __forceinline__ void sweep_m_col_ppm(const StageArgs<CTT>& a, const Grid3& g, int i,
                                                 int t, int seg, int S, double* stg_, int tid) {
   double(*sv)[NV][SWEEP_THREADS] = reinterpret_cast<double(*)[NV][SWEEP_THREADS]>(stg_);
+  // FP32 cells are converted once and stay in a window: two slots, m+2 and m+3
+  constexpr bool kWindow = sizeof(R) == 4;
+  constexpr int RING = kWindow ? 2 : 5;
   double(*sb)[SWEEP_THREADS] =
-      reinterpret_cast<double(*)[SWEEP_THREADS]>(stg_ + 5 * NV * SWEEP_THREADS);
+      reinterpret_cast<double(*)[SWEEP_THREADS]>(stg_ + RING * NV * SWEEP_THREADS);
   const int nd = (DIR == 1) ? g.ny : g.nz;
   const long long n = g.n;
   const R gamma = (R)a.gamma;
@@ -1132,28 +1140,35 @@ __device__ __forceinline__ void sweep_m_col_ppm(const StageArgs<CTT>& a, const G
         cp_async8(&sb[m & 1][tid],
                   a.Bs[DIR] + base + (long long)gidx(m, nd, g.outflow, DIR) * stride);
     };
-    SumStage<PHYS, NV, NDIM, SUM, CTT> ss{a, n, stg_ + (5 * NV + 2) * SWEEP_THREADS, tid};
-    // slots q .. q+3 (mod 5) hold cells m-1 .. m+2
-    stage_cell(m0 - 1, 0);
-    stage_cell(m0, 1);
-    stage_cell(m0 + 1, 2);
-    cp_async_commit();
-    stage_cell(m0 + 2, 3);
+    SumStage<PHYS, NV, NDIM, SUM, CTT> ss{a, n, stg_ + (RING * NV + 2) * SWEEP_THREADS, tid};
+    // FP64: slots q .. q+3 (mod 5) hold cells m-1 .. m+2; window: slot q cell m+2
+    if constexpr (!kWindow) {
+      stage_cell(m0 - 1, 0);
+      stage_cell(m0, 1);
+      stage_cell(m0 + 1, 2);
+      cp_async_commit();
+    }
+    stage_cell(m0 + 2, kWindow ? 0 : 3);
     stage_face(m0);
     cp_async_commit();
-    // FP32 cells are converted once and stay in a window
-    constexpr bool kWindow = sizeof(R) == 4;
     R Fm[NV], vLn[NV], Fp[NV], cmp = R(0), W0[NV], W1[NV], W2[NV];
     {
       R q3[NV], q2[NV], w0[NV];
       load_cell<NV>(a.V, n, base + gidx(m0 - 3, nd, g.outflow, DIR) * stride, q3);
       load_cell<NV>(a.V, n, base + gidx(m0 - 2, nd, g.outflow, DIR) * stride, q2);
-      cp_async_wait1();
+      if constexpr (kWindow) {
+        load_cell<NV>(a.V, n, base + gidx(m0 - 1, nd, g.outflow, DIR) * stride, W0);
+        load_cell<NV>(a.V, n, base + (long long)m0 * stride, W1);
+        load_cell<NV>(a.V, n, base + gidx(m0 + 1, nd, g.outflow, DIR) * stride, W2);
+      } else {
+        cp_async_wait1();
+      }
       R vrp[NV];
 #pragma unroll
       for (int nv = 0; nv < NV; nv++) {
-        const R w1 = (R)sv[1][nv][tid], w2 = (R)sv[2][nv][tid];
-        w0[nv] = (R)sv[0][nv][tid];
+        const R w1 = kWindow ? W1[nv] : (R)sv[1][nv][tid];
+        const R w2 = kWindow ? W2[nv] : (R)sv[2 % RING][nv][tid];
+        w0[nv] = kWindow ? W0[nv] : (R)sv[0][nv][tid];
         const R fa = ppm_face(q3[nv], q2[nv], w0[nv], w1);   // face m0-1
         Fm[nv] = ppm_face(q2[nv], w0[nv], w1, w2);           // face m0
         R dvp, dvm;
@@ -1161,18 +1176,14 @@ __device__ __forceinline__ void sweep_m_col_ppm(const StageArgs<CTT>& a, const G
         vLn[nv] = w0[nv] + dvp;
         vrp[nv] = w0[nv] + dvm;
         Fp[nv] = R(0);
-        if constexpr (kWindow) {
-          W0[nv] = w0[nv];
-          W1[nv] = w1;
-          W2[nv] = w2;
-        }
       }
       if constexpr (PHYS == PHYS_RMHD) rmhd_vel_limit<NV>(w0, vrp, vLn);
     }
     int q = 0;
     for (int m = m0; m <= m1; m++) {
-      const int q1 = q + 1 < 5 ? q + 1 : 0, q2 = q1 + 1 < 5 ? q1 + 1 : 0;
-      const int q3 = q2 + 1 < 5 ? q2 + 1 : 0, q4 = q3 + 1 < 5 ? q3 + 1 : 0;
+      const int q1 = q + 1 < RING ? q + 1 : 0, q2 = q1 + 1 < RING ? q1 + 1 : 0;
+      const int q3 = kWindow ? q : (q2 + 1 < RING ? q2 + 1 : 0);
+      const int q4 = q3 + 1 < RING ? q3 + 1 : 0;
       if (m < m1) {   // prefetch for the next iteration
         stage_cell(m + 3, q4);
         stage_face(m + 1);
@@ -1450,7 +1461,8 @@ __device__ __forceinline__ void sweep_m_col_f32(const StageArgs<CTT>& a, const G
 
 // One (x column i, transverse index t, pencil segment seg) per thread: t is
 // k for DIR=1 and j for DIR=2; the segment covers cells [seg*S, seg*S+S).
-// `stg_` is the block's staging area (sweep_m_stage_doubles<NV>() doubles).
+// `stg_` is the block's staging area (sweep_m_stage_doubles<NV, LIM, R, SUM>()
+// doubles).
 template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, bool SUM, typename R,
           typename CTT>
 __device__ __forceinline__ void sweep_m_col(const StageArgs<CTT>& a, const Grid3& g, int i, int t,
@@ -1586,7 +1598,7 @@ template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR, typename
 __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_m_minb<PHYS, R>()))
     sweep_m_kernel(StageArgs<CTT> a, Grid3 g, int S, bool flat) {
   constexpr bool SUM = sum_directions<PHYS, CTT>();
-  __shared__ double stg[sweep_m_stage_doubles<NV, LIM, SUM>()];
+  __shared__ double stg[sweep_m_stage_doubles<NV, LIM, R, SUM>()];
   step_order();
   const int nd = (DIR == 1) ? g.ny : g.nz;
   const int nseg = (nd + S - 1) / S;
@@ -1624,8 +1636,8 @@ struct SweepSplit {
 template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, bool WHOLE, typename R, typename CTT>
 __global__ void __launch_bounds__(SWEEP_THREADS, (sweeps_minb<PHYS, R>()))
     sweeps_kernel(StageArgs<CTT> a, Grid3 g, SweepSplit sp) {
-  constexpr int nx = sweep_x_stage_doubles<NV, LIM>();
-  constexpr int nm = sweep_m_stage_doubles<NV, LIM>();
+  constexpr int nx = sweep_x_stage_doubles<NV, LIM, R, WHOLE>();
+  constexpr int nm = sweep_m_stage_doubles<NV, LIM, R>();
   __shared__ double stg[nx > nm ? nx : nm];
   step_order();
   int b = sp.first + blockIdx.x, i, t, seg;
