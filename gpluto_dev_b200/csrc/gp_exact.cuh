@@ -23,10 +23,15 @@
 //     would take the step to it.
 //   * q = a y, q + y (a - b q) with y = RN(1/b) is RN(a/b) (no exception while
 //     nothing under- or overflows).
-//   * s + h (a - s^2), s = a y, h = y/2 with y within 0.55 ulp of a^(-1/2) is
-//     RN(sqrt(a)).
-// All three hold for every significand of 4 to 12 bits (checked exhaustively)
-// and agree with the operators on the arguments of tests/test_gpu_exact.py.
+//   * s + h (a - s^2), s = RN(a y), h = y/2 with y within 0.55 ulp of a^(-1/2) is
+//     RN(sqrt(a)) (Markstein's correction of a root).  That y is one step from the
+//     seed y0 with e = 1 - a y0^2: a^(-1/2) = y0 (1 - e)^(-1/2), whose binomial
+//     series is 1 + e/2 + 3 e^2/8 + 5 e^3/16 + ...  The seed holds 21 significand
+//     bits, so y0^2 is exact and e good to 2^-53 |e|; the rounding of y adds 0.5 ulp
+//     and the omitted term 5/16 |e|^3 <= 2^-57.4, or 0.05 ulp, for |e| <= 2^-18.6.
+// All three hold for every significand of 4 to 12 bits (tests/test_exact_small.py);
+// tests/test_gpu_exact.py measures the seeds (|e| up to 2^-19.9 and 2^-19.0, all upper
+// 20 bits) and compares the results with the operators.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>

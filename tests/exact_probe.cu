@@ -21,6 +21,12 @@ __global__ void probe(const double* a, const double* b, double* out, double* ref
   } else if (op == 5) {
     out[i] = f.div_any(a[i], b[i]);
     ref[i] = a[i] / b[i];
+  } else if (op == 6) {  // 1 - b y0 of the reciprocal's seed, 1 - a y0^2 of the root's
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b[i]));
+    out[i] = __fma_rn(-b[i], y, 1.0);
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a[i]));
+    ref[i] = __fma_rn(-a[i], __dmul_rn(y, y), 1.0);
   } else {
     out[i] = gp::fixed_quot(a[i], b[i], gp::fixed_inv(b[i]));
     ref[i] = a[i] / b[i];

@@ -13,7 +13,7 @@ import pytest
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 HERE = os.path.dirname(os.path.abspath(__file__))
-DIV, INV, ROOT, QUOT_POS, FIXED, DIV_ANY = range(6)
+DIV, INV, ROOT, QUOT_POS, FIXED, DIV_ANY, SEEDS = range(7)
 
 
 @pytest.fixture(scope="module")
@@ -105,3 +105,16 @@ def test_special_values(probe):
     for a in (0.0, -0.0, -1.0, tiny, 1e-320, inf, nan, 1e-130, 1e130):
         assert probe([a], [1.0], ROOT)[2].all()
         assert a > 0 or probe([a], [1.0], QUOT_POS)[2].all()
+
+
+def test_seed_errors(probe):
+    """The seeds are as good as gp_exact.cuh's derivation needs: e = 1 - b y0 with
+    |e|^3 <= 2^-58, and e = 1 - a y0^2 with 5/16 |e|^3 <= 2^-57.4 (0.05 ulp of a root's
+    iterate).  They are functions of an argument's upper 20 significand bits: all of
+    those, the rest zero or ones, both parities of the exponent."""
+    top = torch.arange(1 << 20, device="cuda", dtype=torch.int64) << 32
+    m = torch.cat([top, top | 0xffffffff])
+    a = torch.cat([m | (1023 << 52), m | (1024 << 52)]).view(torch.float64)
+    rcp, rsqrt, _ = probe(a, a, SEEDS)
+    assert rcp.abs().max().item() ** 3 <= 2.0 ** -58
+    assert 5.0 / 16.0 * rsqrt.abs().max().item() ** 3 <= 2.0 ** -57.4
