@@ -357,7 +357,7 @@ GP_CR_FN double sqrt_cr(double t) {
 
 // correctly rounded acos(x), -1 <= x <= 1.  asin(s) starts from the FP32
 // function (the FP64 one took a third of this function's time), y0 within
-// 2^-21 of it relative, and takes the inverse sine's Taylor step to third
+// 2^-21 of it relative (2^-22.3 measured, tests/test_gpu_crmath.py), and takes the inverse sine's Taylor step to third
 // order in d = (s - sin y0) / cos y0:
 //   asin s = y0 + d + t/2 d^2 + (1 + 3 t^2)/6 d^3 + O(d^4),  t = tan y0,
 // the neglected term below 2^-83 relative and the step's own roundings below
