@@ -38,18 +38,15 @@
 
 namespace gp {
 
-// The language's operators (FP32 of the mixed form; FP64 where a face left
-// the range of FastArith).
-template <typename R>
+// The language's operators, with the interface of FastArith: the faces that leave
+// its range, and what is not in a sweep.
 struct PlainArith {
   static constexpr bool FAST = false;
-  __device__ __forceinline__ R inv(R b) { return R(1) / b; }
-  __device__ __forceinline__ R inv_pos(R b) { return R(1) / b; }
-  __device__ __forceinline__ R quot(R a, R b, R) { return a / b; }
-  __device__ __forceinline__ R quot_pos(R a, R b, R) { return a / b; }
-  __device__ __forceinline__ R div(R a, R b) { return a / b; }
-  __device__ __forceinline__ R root(R a) { return sqrt(a); }
-  __device__ __forceinline__ R root0(R a) { return sqrt(a); }
+  __device__ __forceinline__ double inv(double b) { return 1.0 / b; }
+  __device__ __forceinline__ double quot(double a, double b, double) { return a / b; }
+  __device__ __forceinline__ double div(double a, double b) { return a / b; }
+  __device__ __forceinline__ double root(double a) { return sqrt(a); }
+  __device__ __forceinline__ double root0(double a) { return sqrt(a); }
 };
 
 struct FastArith {

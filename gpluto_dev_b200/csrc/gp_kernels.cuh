@@ -8,16 +8,19 @@
 // give identical operands, so results agree bit for bit).
 //
 // One RK stage (Src/update_stage.cpp:57-438 + Src/rk_step.cpp:357-593):
-//   sweep_x   : warp per x-row; PLM + Riemann per face, flux difference into
-//               dU (=), per-cell inverse dt into Cdt (=), UCT face data.
-//   sweep_m<d>: thread per (x, pencil segment) marching along y or z with a
-//               register window; dU (+=), Cdt (+=); the last direction fuses
-//               the RK combine (writes U_out) and the stage-1 CFL max.
+//   sweep x   : warp per x-row or part of one; reconstruction + Riemann per face,
+//               flux difference into dU, per-cell inverse dt into Cdt, UCT face data.
+//   sweep y, z: thread per (x, pencil segment) marching along the direction, the
+//               same outputs.  Each direction writes arrays of its own (FP64 HD: one
+//               array that y and z add to); MHD and mixed HD sweep all directions
+//               in one launch (sweeps_kernel), RMHD and FP64 HD in one each.
 //   emf       : thread per cell, its three edge EMFs (UCT_HLLD / UCT_HLL
 //               composition, Src/MHD/CT/ct_emf_average.cpp:535-995).
 //   finish    : thread per cell: CT face update of its left faces (and the
 //               right faces recomputed for the cell average), RK combine of
-//               the faces, cell-centred B average, con2prim -> V, U fixups.
+//               the faces, cell-centred B average, sum of the directions' flux
+//               differences and RK combine of U, con2prim -> V, U fixups, the
+//               stage-1 CFL maximum (per warp).
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -1064,11 +1067,11 @@ __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_x_minb<PHYS, R>()))
 }
 
 // ---------------------------------------------------------------------
-// y / z sweep: thread per (x, pencil segment), marching along DIR with a
-// register window of three cells; the cell two steps ahead and the next face
-// field are staged into shared memory with cp.async while the current face
-// is solved.  Writes the direction's flux differences, inverse-dt terms and
-// UCT face data (no loads besides the stencil).
+// y / z sweep: thread per (x, pencil segment), marching along DIR.  Cells and face
+// fields are staged into shared memory with cp.async while the current face is
+// solved: FP64 keeps the stencil there (a ring of cells), FP32 in a register window
+// fed from two slots.  Writes the direction's flux differences, inverse-dt terms and
+// UCT face data.
 // ---------------------------------------------------------------------
 // The flux differences and inverse-dt term the directions before left in a
 // cell, staged into shared memory an iteration before they are added to
@@ -2425,7 +2428,7 @@ __device__ __forceinline__ double finish_cell(const StageArgs<CTT>& a, const Gri
     uint32_t le;
     if constexpr (PHYS == PHYS_MHD) le = mhd_cons2prim(u, v, a.gamma, a.small_rho, a.small_prs);
     else if constexpr (PHYS == PHYS_RMHD) {
-      PlainArith<double> ar;
+      PlainArith ar;
       le = rmhd_cons2prim(u, v, a.gamma, a.small_rho, a.small_prs, ar);
     }
     else le = hd_cons2prim(u, v, a.gamma, a.small_rho, a.small_prs);

@@ -470,8 +470,9 @@ __device__ __forceinline__ void ct_store_ucthlld(const R* ul, const R* ur, const
 
 // mhd_prim2cons and the signal speeds with the divisions and roots of `ar`
 // (y = 1/(gamma - 1)); same expressions, so the same values
-template <typename R, typename A>
-__device__ __forceinline__ void mhd_prim2cons(const R* v, R* u, R gmm1, R y, A& ar) {
+__device__ __forceinline__ void mhd_prim2cons(const double* v, double* u, double gmm1, double y,
+                                              FastArith& ar) {
+  using R = double;
   u[RHO] = v[RHO];
   u[MX1] = v[RHO] * v[VX1];
   u[MX2] = v[RHO] * v[VX1 + 1];
@@ -485,8 +486,10 @@ __device__ __forceinline__ void mhd_prim2cons(const R* v, R* u, R gmm1, R y, A& 
   u[7] = kinb2 + ar.quot_bpos(v[7], gmm1, y);  // p > 0 in range, as gamma p is
 }
 
-template <int DIR, typename R, typename A>
-__device__ __forceinline__ void mhd_signal_speed(const R* v, R gamma, R& cmin, R& cmax, A& ar) {
+template <int DIR>
+__device__ __forceinline__ void mhd_signal_speed(const double* v, double gamma, double& cmin,
+                                                 double& cmax, FastArith& ar) {
+  using R = double;
   constexpr int VXn = VX1 + DIR;
   const R yr = ar.inv_pos(v[RHO]);
   const R a2 = ar.quot_pos(gamma * v[7], v[RHO], yr);
@@ -508,9 +511,11 @@ __device__ __forceinline__ void mhd_signal_speed(const R* v, R gamma, R& cmin, R
 // becomes one selection of the side, and the physical flux, the star energy
 // and the double-star state are formed for that side only.  Every value kept
 // is the one mhd_hlld computes.
-template <int DIR, int CT, typename R, typename A>
-__device__ __forceinline__ R mhd_hlld_line(const R* vl, const R* vr, R* flux, R gamma, R ygm,
-                                           R Bn, CTFace<R>& ct, A& ar) {
+template <int DIR, int CT>
+__device__ __forceinline__ double mhd_hlld_line(const double* vl, const double* vr, double* flux,
+                                                double gamma, double ygm, double Bn,
+                                                CTFace<double>& ct, FastArith& ar) {
+  using R = double;
   constexpr int VXn = VX1 + DIR, VXt = VX1 + (DIR + 1) % 3, VXb = VX1 + (DIR + 2) % 3;
   constexpr int MXn = MX1 + DIR, MXt = MX1 + (DIR + 1) % 3, MXb = MX1 + (DIR + 2) % 3;
   constexpr int BXn = BX1 + DIR, BXt = BX1 + (DIR + 1) % 3, BXb = BX1 + (DIR + 2) % 3;
@@ -1170,9 +1175,10 @@ __device__ __forceinline__ R hd_hllc(const R* vl, const R* vr, R* flux, R gamma)
 // hd_hllc for faces FastArith covers, in straight-line form: the side is
 // selected first, and the flux and star state formed for it alone (ygm =
 // 1/(gamma - 1)).  Every value kept is the one hd_hllc computes.
-template <int DIR, typename R, typename A>
-__device__ __forceinline__ R hd_hllc_line(const R* vl, const R* vr, R* flux, R gamma, R ygm,
-                                          A& ar) {
+template <int DIR>
+__device__ __forceinline__ double hd_hllc_line(const double* vl, const double* vr, double* flux,
+                                               double gamma, double ygm, FastArith& ar) {
+  using R = double;
   constexpr int VXn = VX1 + DIR, VXt = VX1 + (DIR + 1) % 3, VXb = VX1 + (DIR + 2) % 3;
   constexpr int MXn = MX1 + DIR, MXt = MX1 + (DIR + 1) % 3, MXb = MX1 + (DIR + 2) % 3;
   const R yl = ar.inv_pos(vl[RHO]), yr = ar.inv_pos(vr[RHO]);

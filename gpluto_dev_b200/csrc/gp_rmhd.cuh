@@ -57,7 +57,7 @@ __device__ __forceinline__ void rmhd_prim2cons(const R* v, R* u, R gmmr, R h, A&
 
 // the start-up map
 __device__ __forceinline__ void rmhd_prim2cons(const double* v, double* u, double gamma) {
-  PlainArith<double> ar;
+  PlainArith ar;
   const double gmmr = gamma / (gamma - 1.0);
   rmhd_prim2cons(v, u, gmmr, rmhd_enthalpy(v, gmmr, 0.0, ar), ar);
 }
@@ -742,7 +742,7 @@ __device__ __noinline__ uint32_t rmhd_riemann_call(double* io) {
   double flux[8];
   CTFace<double> ct;
   uint32_t err = 0;
-  PlainArith<double> ar;
+  PlainArith ar;
   const double cmax = rmhd_riemann<DIR, RS>(io, io + 8, flux, io[16], ct, err, ar);
   face_out(io, flux, ct, cmax);
   return err;
