@@ -139,8 +139,8 @@ constexpr int SWEEP_THREADS = 128;
 // All sweeps in one kernel (sweeps_kernel: MHD, mixed HD).  FP64 at 3 (168
 // registers): 1000^2 four steps 1755 us, 100^3 2847; at 2, without spills, 1816
 // and 2972 (256^2 ten steps 643 and 608).  FP32 MHD at 4 (126): 333x171 ten steps
-// 505 us, 64^3 PPM four steps 782, 200^3 12723; at 5 518, 822 and 12628.  FP32 HD
-// at 5: 384^2 four steps 174 us (at 4 183).
+// 505 us, 64^3 PPM four steps 782, 512^2 PPM 767, 200^3 12723; at 5 518, 822, 827 and
+// 12628.  FP32 HD at 5: 384^2 four steps 174 us (at 4 183).
 template <int PHYS, typename R>
 constexpr int sweeps_minb() {
   return sizeof(R) == 8 ? 3 : (PHYS == PHYS_MHD ? 4 : 5);

@@ -79,21 +79,45 @@ constexpr bool one_sweep_launch(int physics, bool mixed) {
   return physics == PHYS_MHD || (physics == PHYS_HD && mixed);
 }
 
-// Launch in stream order, on a grid of at most kEarlyCells cells with its blocks
-// placed while the kernel before drains (step_order)
+// How the kernels of a stage are launched.
+struct How {
+  bool early;  // blocks placed while the kernel before drains (step_order)
+  int split;   // percent of an SM's memory that is shared memory (0: the driver's choice)
+};
+
+// Where two kernels in a row want different splits, the second one's blocks wait
+// until the SM is empty.  FP32 MP5 and WENO-Z in 3-D do (sweeps 4 blocks of 35 KB, EMF
+// tiles 3 of 54 KB, finish none), and on small grids that costs more than an EMF block
+// fewer: with the sweeps' split for all, MP5 32^3 190 -> 135 us a step, 48^3 263 -> 229,
+// 64^3 370 -> 340, WENO-Z 272 -> 251; from 2^18 cells on it loses (MP5 64x64x80 416 ->
+// 426, 80^3 612 -> 631).
+template <int PHYS, int NDIM, int LIM>
+static How how_to_launch(long long cells) {
+  const bool fix = PHYS == PHYS_MHD && NDIM == 3 && sizeof(RT) == 4 && five_point<LIM>();
+  return How{cells <= kEarlyCells, fix && cells <= (1LL << 18) ? 64 : 0};
+}
+
+// Launch in stream order
 template <typename... K, typename... A>
-static void launch(long long cells, void (*k)(K...), dim3 grid, dim3 block, size_t smem,
-                   cudaStream_t s, A... args) {
-  cudaLaunchAttribute early;
-  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  early.val.programmaticStreamSerializationAllowed = 1;
+static void launch(How how, void (*k)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                   A... args) {
+  cudaLaunchAttribute at[2];
+  unsigned n = 0;
+  if (how.early) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (how.split) {
+    at[n].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at[n++].val.sharedMemCarveout = how.split;
+  }
   cudaLaunchConfig_t c = {};
   c.gridDim = grid;
   c.blockDim = block;
   c.dynamicSmemBytes = smem;
   c.stream = s;
-  c.attrs = &early;
-  c.numAttrs = cells <= kEarlyCells ? 1 : 0;
+  c.attrs = at;
+  c.numAttrs = n;
   cudaLaunchKernelEx(&c, k, K(args)...);
 }
 
@@ -146,12 +170,13 @@ static int march_length(long long cols, int nd, int blocks_per_sm) {
 // block (sweep_m_kernel)
 template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, int DIR>
 static void launch_m(const StageArgs<CTT>& a, const Grid3& g, int nt, int nd, cudaStream_t s) {
+  const How how = how_to_launch<PHYS, NDIM, LIM>(g.n);
   const long long cols = ((long long)g.nx * nt + SWEEP_THREADS - 1) / SWEEP_THREADS;
   const int seg = march_length(cols, nd, sweep_m_minb<PHYS, RT>());
   const int nseg = (nd + seg - 1) / seg;
   const bool flat = g.nx % SWEEP_THREADS != 0 || (long long)nt * nseg > 65535;
   const dim3 grid = flat ? dim3((unsigned)(cols * nseg)) : dim3(g.nx / SWEEP_THREADS, nt * nseg);
-  launch(g.n, sweep_m_kernel<PHYS, NV, NDIM, RS, CT, LIM, DIR, RT, CTT>, grid, SWEEP_THREADS, 0, s,
+  launch(how, sweep_m_kernel<PHYS, NV, NDIM, RS, CT, LIM, DIR, RT, CTT>, grid, SWEEP_THREADS, 0, s,
          a, g, seg, flat);
 }
 
@@ -167,6 +192,7 @@ template <int PHYS, int NV, int NDIM, int RS, int CT, int LIM, typename F1, type
 static void launch_sweeps(const StageArgs<CTT>& a, const Grid3& g, cudaStream_t s, bool each,
                           F1& pre, F2& post) {
   constexpr int per_sm = sweeps_minb<PHYS, RT>();
+  const How how = how_to_launch<PHYS, NDIM, LIM>(g.n);
   const long long rows = (long long)g.ny * g.nz;
   SweepSplit sp = {};
   sp.xseg = x_segments<LIM>(g.nx, rows, per_sm);
@@ -185,10 +211,10 @@ static void launch_sweeps(const StageArgs<CTT>& a, const Grid3& g, cudaStream_t 
     // FP32 rows in one part keep their shuffles and carry (256^3: 546 us against
     // 600 through shared memory, which is what parts of rows need)
     if (whole_row_form<LIM, RT>() && sp.xseg == 1)
-      launch(g.n, sweeps_kernel<PHYS, NV, NDIM, RS, CT, LIM, whole_row_form<LIM, RT>(), RT, CTT>,
+      launch(how, sweeps_kernel<PHYS, NV, NDIM, RS, CT, LIM, whole_row_form<LIM, RT>(), RT, CTT>,
              count, SWEEP_THREADS, 0, s, a, g, sp);
     else
-      launch(g.n, sweeps_kernel<PHYS, NV, NDIM, RS, CT, LIM, false, RT, CTT>, count, SWEEP_THREADS,
+      launch(how, sweeps_kernel<PHYS, NV, NDIM, RS, CT, LIM, false, RT, CTT>, count, SWEEP_THREADS,
              0, s, a, g, sp);
     post();
   };
@@ -211,6 +237,7 @@ static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, cudaStream_t 
     g.glo[d] = gd.glo[d];
     g.ghi[d] = gd.ghi[d];
   }
+  const How how = how_to_launch<PHYS, NDIM, LIM>(gd.n);
   int kidx = 0;
   auto pre = [&]() { if (ev) cudaEventRecord(ev[2 * kidx], s); };
   auto post = [&]() { if (ev) cudaEventRecord(ev[2 * kidx + 1], s); kidx++; };
@@ -223,10 +250,10 @@ static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, cudaStream_t 
     const unsigned grid = x_blocks(rows, nseg);
     pre();
     if (whole_row_form<LIM, RT>() && nseg == 1)
-      launch(gd.n, sweep_x_kernel<PHYS, NV, NDIM, RS, CT, LIM, whole_row_form<LIM, RT>(), RT, CTT>,
+      launch(how, sweep_x_kernel<PHYS, NV, NDIM, RS, CT, LIM, whole_row_form<LIM, RT>(), RT, CTT>,
              grid, SWEEP_THREADS, 0, s, a, g, nseg);
     else
-      launch(gd.n, sweep_x_kernel<PHYS, NV, NDIM, RS, CT, LIM, false, RT, CTT>, grid, SWEEP_THREADS,
+      launch(how, sweep_x_kernel<PHYS, NV, NDIM, RS, CT, LIM, false, RT, CTT>, grid, SWEEP_THREADS,
              0, s, a, g, nseg);
     post();
     pre();
@@ -242,9 +269,9 @@ static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, cudaStream_t 
   if constexpr (PHYS != PHYS_HD) {
     pre();
     if constexpr (CT == CT_ARITH) {
-      launch(gd.n, emf_arith_kernel<NDIM, RT, CTT>, nb, 256, 0, s, a, g);
+      launch(how, emf_arith_kernel<NDIM, RT, CTT>, nb, 256, 0, s, a, g);
     } else if constexpr (CT == CT_CONTACT) {
-      launch(gd.n, emf_contact_kernel<NDIM, RT, CTT>, nb, 256, 0, s, a, g);
+      launch(how, emf_contact_kernel<NDIM, RT, CTT>, nb, 256, 0, s, a, g);
     } else if constexpr (NDIM == 3 && (sizeof(RT) == 8 || five_point<LIM>())) {  // plane-staged EMF
       using T = EmfTile<LIM, CTT>;
       cudaFuncSetAttribute(emf_tile_kernel<LIM, RT, CTT>,
@@ -255,7 +282,7 @@ static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, cudaStream_t 
       int sz = ET_SEGMENT;
       while (sz > 4 && cols * ((gd.nz + sz - 1) / sz) < 148LL * emf_tile_minb<RT>() * 4) sz /= 2;
       dim3 grid((gd.nx + ETX - 1) / ETX, (gd.ny + ETY - 1) / ETY, (gd.nz + sz - 1) / sz);
-      launch(gd.n, emf_tile_kernel<LIM, RT, CTT>, grid, dim3(ETX, ETY), T::SMEM, s, a, g, sz);
+      launch(how, emf_tile_kernel<LIM, RT, CTT>, grid, dim3(ETX, ETY), T::SMEM, s, a, g, sz);
     } else if constexpr (NDIM == 3) {  // mixed PLM/PPM: z-marching EMF, loads through L1
       // the longest segment (<= EMF_SEGMENT planes) that still gives about
       // four waves of blocks over 148 SMs (3 blocks per SM)
@@ -265,14 +292,14 @@ static void run_stage(const StageArgs<CTT>& a, const GridDims& gd, cudaStream_t 
       while (sz > 4 && cols * ((gd.nz + sz - 1) / sz) < 148LL * 3 * 4) sz /= 2;
       dim3 grid((gd.nx + EMF_TX - 1) / EMF_TX, (gd.ny + EMF_TY - 1) / EMF_TY,
                 (gd.nz + sz - 1) / sz);
-      launch(gd.n, emf_march_kernel<LIM, RT, CTT>, grid, dim3(EMF_TX, EMF_TY), 0, s, a, g, sz);
+      launch(how, emf_march_kernel<LIM, RT, CTT>, grid, dim3(EMF_TX, EMF_TY), 0, s, a, g, sz);
     } else {
-      launch(gd.n, emf_kernel<NDIM, LIM, RT, CTT>, nb, 256, 0, s, a, g);
+      launch(how, emf_kernel<NDIM, LIM, RT, CTT>, nb, 256, 0, s, a, g);
     }
     post();
   }
   pre();
-  launch(gd.n, finish_kernel<PHYS, NV, NDIM, CTT>, nb, 256, 0, s, a, g);
+  launch(how, finish_kernel<PHYS, NV, NDIM, CTT>, nb, 256, 0, s, a, g);
   post();
 }
 
