@@ -1628,10 +1628,11 @@ __global__ void __launch_bounds__(SWEEP_THREADS, (sweep_m_minb<PHYS, R>()))
 // mixed 6100 -> 6097.  RMHD keeps one launch a sweep (90x72x60 lost 12%: two long
 // codes in one instruction cache), and so do the forms whose sweeps add up in one
 // array.
-// Blocks [0, nb[0]) sweep z, the next nb[1] y, the rest x; `first` is the number of
-// the launch's first block, so that one direction can be launched (and timed) alone.
+// Blocks [0, nb[0]) sweep z, the next nb[1] y, the rest up to `total` x; `first` is the
+// number of the launch's first block, wrapped at `total`, so that x can come first and
+// one direction can be launched (and timed) alone.
 struct SweepSplit {
-  int first;
+  int first, total;
   int xseg, len[2];  // parts of an x-row, march lengths (y, z)
   int nb[2];         // blocks (z, y)
 };
@@ -1644,6 +1645,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS, (sweeps_minb<PHYS, R>()))
   __shared__ double stg[nx > nm ? nx : nm];
   step_order();
   int b = sp.first + blockIdx.x, i, t, seg;
+  if (b >= sp.total) b -= sp.total;
   if constexpr (NDIM == 3) {
     if (b < sp.nb[0]) {
       flat_column(g.nx, g.ny, (unsigned)((g.nz + sp.len[1] - 1) / sp.len[1]), b, i, t, seg);
