@@ -100,3 +100,27 @@ def test_overlapped_sweeps_match_serialized_launches(physics, n, precision):
     b.profile(40, 1e-4)
     for x, y in zip(a.download(), b.download()):
         np.testing.assert_array_equal(np.asarray(x), np.asarray(y))
+
+
+@pytest.mark.parametrize("n, limiter", [((420, 300), "ppm"), ((500, 330), "mp5"),
+                                        ((200, 20, 60), "wenoz")])
+def test_x_rows_first(n, limiter):
+    """Uncut rows that are the longest chains of a launch whose blocks do not all fit
+    (the 2-D grids) come first, wrapped round the marches; the 3-D one does not wrap."""
+    gen = ics.mhd2d_turbulence if len(n) == 2 else ics.mhd3d_turbulence
+    check(gen(n=n, seed=sum(n)), limiter=limiter, nsteps=2)
+
+
+@pytest.mark.parametrize("n, limiter", [((1100, 420), "ppm"), ((1100, 420), "wenoz"),
+                                        ((20, 16, 12), "mp5"), ((36, 30, 44), "wenoz")])
+def test_common_launch_matches_one_a_direction(n, limiter):
+    """The same in FP32, where the profiled launches (one direction each, of the same
+    kernel) give the bits; small 3-D grids of these forms also fix the memory split."""
+    gen = ics.mhd2d_turbulence if len(n) == 2 else ics.mhd3d_turbulence
+    st = gen(n=n, seed=7)
+    sch = api.Scheme(physics=st.physics, limiter=limiter, gamma=st.gamma, precision=api.MIXED)
+    a, b = api.Solver.from_state(st, sch), api.Solver.from_state(st, sch)
+    a.run(6, 1e-4)
+    b.profile(6, 1e-4)
+    for x, y in zip(a.download(), b.download()):
+        np.testing.assert_array_equal(np.asarray(x), np.asarray(y))
